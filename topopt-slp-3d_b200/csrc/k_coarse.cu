@@ -449,49 +449,21 @@ template void launch_stencil<float>(const float *, const float *, const float *,
                                     const Grid &, int, bool, cudaStream_t);
 
 // ---------------------------------------------------------------------------
-// Elementwise smoother pieces for the matrix-free finest level.
+// Elementwise smoother pieces.
 // ---------------------------------------------------------------------------
+// First sweep from a zero guess, x = invD b (b - A*0 = b exactly, so the
+// product is skipped).
 template <typename T>
-__global__ void k_residual(const T *b, const T *t, T *r, int64_t n) {
+__global__ void k_jacobi_zero(T *x, const T *b, const T *invd, int64_t n) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        r[i] = b[i] - t[i];
+        x[i] = invd[i] * b[i];
 }
 template <typename T>
-void launch_residual(const T *b, const T *t, T *r, int64_t n, cudaStream_t st) {
-    k_residual<T><<<grid_for(n, 256), 256, 0, st>>>(b, t, r, n); count_launch();
+void launch_jacobi_zero(T *x, const T *b, const T *invdiag, int64_t n, cudaStream_t st) {
+    k_jacobi_zero<T><<<grid_for(n, 256), 256, 0, st>>>(x, b, invdiag, n); count_launch();
 }
-template void launch_residual<double>(const double *, const double *, double *, int64_t, cudaStream_t);
-template void launch_residual<float>(const float *, const float *, float *, int64_t, cudaStream_t);
-
-// x = x + invD (b - t), or x = invD b for the first sweep from a zero guess
-// (b - A*0 = b exactly, so the product is skipped).
-template <typename T>
-__global__ void k_jacobi(T *x, const T *b, const T *t, const T *invd, int64_t n, int first) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        x[i] = first ? invd[i] * b[i] : x[i] + invd[i] * (b[i] - t[i]);
-}
-template <typename T>
-void launch_jacobi_update(T *x, const T *b, const T *t, const T *invdiag, int64_t n, int first, cudaStream_t st) {
-    k_jacobi<T><<<grid_for(n, 256), 256, 0, st>>>(x, b, t, invdiag, n, first); count_launch();
-}
-template void launch_jacobi_update<double>(double *, const double *, const double *, const double *, int64_t, int,
-                                           cudaStream_t);
-template void launch_jacobi_update<float>(float *, const float *, const float *, const float *, int64_t, int,
-                                          cudaStream_t);
-
-template <typename T>
-__global__ void k_jacobi_out(double *out, const T *x, const T *b, const T *t, const T *invd, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = (double)(x[i] + invd[i] * (b[i] - t[i]));
-}
-template <typename T>
-void launch_jacobi_out(double *out, const T *x, const T *b, const T *t, const T *invdiag, int64_t n, cudaStream_t st) {
-    k_jacobi_out<T><<<grid_for(n, 256), 256, 0, st>>>(out, x, b, t, invdiag, n); count_launch();
-}
-template void launch_jacobi_out<double>(double *, const double *, const double *, const double *, const double *,
-                                        int64_t, cudaStream_t);
-template void launch_jacobi_out<float>(double *, const float *, const float *, const float *, const float *, int64_t,
-                                       cudaStream_t);
+template void launch_jacobi_zero<double>(double *, const double *, const double *, int64_t, cudaStream_t);
+template void launch_jacobi_zero<float>(float *, const float *, const float *, int64_t, cudaStream_t);
 
 template <typename T>
 __global__ void k_invert_diag(const T *diag, const uint8_t *fm, T *invd, double omega, int64_t n) {
@@ -566,11 +538,10 @@ template void launch_prolong<double>(const double *, double *, const uint8_t *, 
 template void launch_prolong<float>(const float *, float *, const uint8_t *, const Grid &, const Grid &, bool,
                                     cudaStream_t);
 
-// RES: restrict rf - tf, the residual b - A x of the finest level.  The 27
-// fine neighbours are read with clamped indices, those outside the mesh
+// The 27 fine neighbours are read with clamped indices, those outside the mesh
 // weighted by zero (loads issue together; same sum, same order).
-template <typename T, bool RES>
-__global__ void k_restrict(const T *__restrict__ rf, const T *__restrict__ tf, T *__restrict__ bc,
+template <typename T>
+__global__ void k_restrict(const T *__restrict__ rf, T *__restrict__ bc,
                            const uint8_t *__restrict__ fmc, Grid gf, Grid gc, const T *__restrict__ invdc,
                            T *__restrict__ xc) {
     for (int64_t J = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; J < gc.nnodes;
@@ -597,15 +568,9 @@ __global__ void k_restrict(const T *__restrict__ rf, const T *__restrict__ tf, T
                                      ? (dx ? T(0.5) : T(1)) * (dy ? T(0.5) : T(1)) * (dz ? T(0.5) : T(1))
                                      : T(0);
                     const int64_t I = ((int64_t)fzc * gf.nx + fxc) * gf.ny + fyc;
-                    if constexpr (RES) {
-                        v0 += wt * (rf[3 * I] - tf[3 * I]);
-                        v1 += wt * (rf[3 * I + 1] - tf[3 * I + 1]);
-                        v2 += wt * (rf[3 * I + 2] - tf[3 * I + 2]);
-                    } else {
-                        v0 += wt * rf[3 * I];
-                        v1 += wt * rf[3 * I + 1];
-                        v2 += wt * rf[3 * I + 2];
-                    }
+                    v0 += wt * rf[3 * I];
+                    v1 += wt * rf[3 * I + 1];
+                    v2 += wt * rf[3 * I + 2];
                 }
             }
         }
@@ -620,19 +585,9 @@ __global__ void k_restrict(const T *__restrict__ rf, const T *__restrict__ tf, T
 template <typename T>
 void launch_restrict(const T *rf, T *bc, const uint8_t *freemask_c, const Grid &gf, const Grid &gc, cudaStream_t st,
                      const T *invd_c, T *xc) {
-    k_restrict<T, false><<<grid_for(gc.nnodes, 256), 256, 0, st>>>(rf, nullptr, bc, freemask_c, gf, gc, invd_c, xc);
+    k_restrict<T><<<grid_for(gc.nnodes, 256), 256, 0, st>>>(rf, bc, freemask_c, gf, gc, invd_c, xc);
     count_launch();
 }
-template <typename T>
-void launch_restrict_res(const T *bf, const T *tf, T *bc, const uint8_t *freemask_c, const Grid &gf, const Grid &gc,
-                         cudaStream_t st, const T *invd_c, T *xc) {
-    k_restrict<T, true><<<grid_for(gc.nnodes, 256), 256, 0, st>>>(bf, tf, bc, freemask_c, gf, gc, invd_c, xc);
-    count_launch();
-}
-template void launch_restrict_res<double>(const double *, const double *, double *, const uint8_t *, const Grid &,
-                                          const Grid &, cudaStream_t, const double *, double *);
-template void launch_restrict_res<float>(const float *, const float *, float *, const uint8_t *, const Grid &,
-                                         const Grid &, cudaStream_t, const float *, float *);
 template void launch_restrict<double>(const double *, double *, const uint8_t *, const Grid &, const Grid &,
                                       cudaStream_t, const double *, double *);
 template void launch_restrict<float>(const float *, float *, const uint8_t *, const Grid &, const Grid &,

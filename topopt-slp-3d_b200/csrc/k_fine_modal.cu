@@ -1,0 +1,531 @@
+// Finest-level operator y = K(w) x (I/WOK/KelemProd.m:57-100) in modal form
+// (fine_modal.cuh), FP64 and FP32, MR factors 1, 2 and 3, any mesh.
+//
+// A block owns a tile of TX x TY node columns and marches along z over LZ node
+// planes; a thread holds one of the EX x EY = (TX + 1) x (TY + 1) element
+// columns that touch the tile.  Per element layer a thread transforms its four
+// nodes of the new plane to plane modes (those of the old plane are still in
+// registers), forms the element's gradient, keeps the part that belongs to
+// the upper plane for the next layer and writes the four corner values of the
+// lower plane to shared memory; after the block's barrier the threads of the
+// owned nodes sum the four columns' corners.  Every node is summed by one
+// thread in a fixed order and written once: no atomics, no zeroing of y, and
+// results are the same from run to run.  The elements at the tile's low edges
+// are computed by two blocks (about 15 % of the work); elements outside the
+// mesh carry zero factors.
+//
+// What the caller does with K x (FineMode) happens where the sums are at hand,
+// so no product vector goes through memory.  The sums pass through shared
+// memory once more, into the order of the global vector, so that the operands
+// and the result are read and written in whole sectors.
+//
+// The node planes, the factors and the operands of the epilogue come by
+// cp.async, one layer ahead of their use.  One barrier per layer: planes,
+// corners and sums are double-buffered.
+#include <cuda_bf16.h>
+
+#include <algorithm>
+#include <cmath>
+
+#include "fine_modal.cuh"
+#include "tosp_internal.h"
+
+namespace tosp {
+
+namespace {
+
+// Threads per block and blocks per SM the registers are capped for.  FP64 keeps
+// 2 x 12 plane modes, 21 modes and 21 gradients in registers (253 for n = 2; a
+// cap of 168 spills, 152 against 119 us at 192 x 96 x 96; n = 1 fits in 160:
+// 80 against 95 us).  FP32 takes 128 (a cap of 80 spills: 131 against 85 us).
+template <typename T> constexpr int fine_threads = sizeof(T) == 8 ? 128 : 256;
+constexpr int fine_resident(int n, int elem_bytes) { return n == 1 && elem_bytes == 8 ? 3 : 2; }
+// Layers per loop trip: two for n = 1, whose carried planes change registers
+// instead of being moved (57 against 62 us, 192 x 96 x 96, BF16); the longer
+// bodies of n = 2 and 3 gain nothing or lose (n = 3: 70 against 57 us).
+constexpr int fine_unroll(int n) { return n == 1 ? 2 : 1; }
+__device__ __forceinline__ float factor_value(__nv_bfloat16 v) { return __bfloat162float(v); }
+__device__ __forceinline__ float factor_value(float v) { return v; }
+__device__ __forceinline__ double factor_value(double v) { return v; }
+
+constexpr uint32_t FINE_NONE = 0xffffffffu;   // no value at this place
+constexpr int FINE_NQ = 4;   // plane values staged per thread
+
+template <int NB>
+__device__ __forceinline__ void cp_async(void *dst, const void *src, bool in) {
+    if constexpr (NB == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                     "l"(src), "r"(in ? NB : 0)
+                     : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                     "l"(src), "n"(NB), "r"(in ? NB : 0)
+                     : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+// The n^3 factors of an element whose first cell is at w (rows along y): each
+// thread stages its own element's into its own slots (slot q of thread t at
+// q * threads + t), so no barrier stands between the copy and the read.  The
+// two cells of a row are one aligned piece for n = 2 (n * nely is even).
+// cp.async moves 4 bytes or more, and 27 of them a layer cost more than they
+// hide (n = 3, 160 x 80 x 40, FP64: 90 against 80 us): BF16 factors of n = 1 and
+// all of n = 3 are read directly, after a prefetch into L2 a layer ahead.
+template <int N, typename WT> constexpr bool fine_stage_w = N == 2 || (N == 1 && sizeof(WT) >= 4);
+template <int N, typename WT>
+struct FineSlot {
+    static constexpr int CELLS = N == 2 ? 2 : 1, BYTES = CELLS * (int)sizeof(WT);
+};
+
+template <int N, typename WT, int TH>
+__device__ __forceinline__ void stage_factors(unsigned char *slots, const WT *w, int64_t row, int64_t plane, bool in) {
+    using S = FineSlot<N, WT>;
+#pragma unroll
+    for (int sz = 0; sz < N; ++sz)
+#pragma unroll
+        for (int sx = 0; sx < N; ++sx) {
+            const WT *p = w + sz * plane + sx * row;
+            if constexpr (fine_stage_w<N, WT>) {
+#pragma unroll
+                for (int sy = 0; sy < N / S::CELLS; ++sy)
+                    cp_async<S::BYTES>(slots + ((sz * N + sx) * (N / S::CELLS) + sy) * TH * S::BYTES, in ? p + sy * S::CELLS : p, in);
+            } else if (in) {
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+            }
+        }
+}
+template <int N, typename T, typename WT, int TH>
+__device__ __forceinline__ void load_factors(const unsigned char *slots, const WT *w, int64_t row, int64_t plane,
+                                             bool in, T (&v)[N * N * N]) {
+    using S = FineSlot<N, WT>;
+#pragma unroll
+    for (int sz = 0; sz < N; ++sz)
+#pragma unroll
+        for (int sx = 0; sx < N; ++sx)
+#pragma unroll
+            for (int sy = 0; sy < N / S::CELLS; ++sy) {
+                const int q = (sz * N + sx) * (N / S::CELLS) + sy;
+                T *o = v + q * S::CELLS;
+                const unsigned char *p = slots + q * TH * S::BYTES;
+                if constexpr (!fine_stage_w<N, WT>) {
+                    o[0] = in ? (T)factor_value(__ldg(w + sz * plane + sx * row + sy)) : T(0);
+                } else if constexpr (N == 2 && sizeof(WT) == 2) {
+                    const __nv_bfloat162 c = *reinterpret_cast<const __nv_bfloat162 *>(p);
+                    o[0] = (T)__low2float(c);
+                    o[1] = (T)__high2float(c);
+                } else if constexpr (N == 2 && sizeof(WT) == 4) {
+                    const float2 c = *reinterpret_cast<const float2 *>(p);
+                    o[0] = (T)c.x;
+                    o[1] = (T)c.y;
+                } else if constexpr (N == 2) {
+                    const double2 c = *reinterpret_cast<const double2 *>(p);
+                    o[0] = (T)c.x;
+                    o[1] = (T)c.y;
+                } else {
+                    o[0] = (T)*reinterpret_cast<const WT *>(p);
+                }
+            }
+}
+
+__device__ __forceinline__ double fine_block_sum(double v, double *sh) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double s = 0.0;
+    if (threadIdx.x == 0)
+        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += sh[i];
+    __syncthreads();
+    return s;   // valid in thread 0
+}
+
+// Bytes of the epilogue's operands per value, in the order of their slots.
+template <typename T, int MODE>
+constexpr int fine_epi_bytes = MODE == FINE_RESID    ? (int)sizeof(T)
+                               : MODE == FINE_JACOBI ? 3 * (int)sizeof(T)
+                               : MODE == FINE_OUT    ? 16 + 2 * (int)sizeof(T)
+                               : MODE == FINE_DOT    ? 8
+                                                     : 0;
+
+template <int N, typename T, typename WT, int MODE>
+size_t fine_smem(const FinePlan &p) {
+    const size_t pl = (size_t)(p.ex + 1) * (p.ey + 1) * 3;
+    const size_t plane = (pl * sizeof(T) + 15) / 16 * 16;
+    return 2 * plane + fine_threads<T> * (2 * 9 * sizeof(T) + 2 * 3 * sizeof(T) + 3 * fine_epi_bytes<T, MODE> +
+                                          (fine_stage_w<N, WT> ? N * N * N * sizeof(WT) : 0));
+}
+
+}  // namespace
+
+template <int N, typename T, typename WT, int MODE>
+__global__ void __launch_bounds__(fine_threads<T>, fine_resident(N, sizeof(T)))
+k_fine_modal(const FineArgs<T> a, const WT *__restrict__ w, const Grid g, const int nelx_d, const int nely_d,
+             const FinePlan pl, const ModalCoef<T> k) {
+    constexpr int TH = fine_threads<T>, SZ = (int)sizeof(T), UNROLL = fine_unroll(N);
+    constexpr bool MASK = MODE == FINE_APPLY || MODE == FINE_RESID || MODE == FINE_DOT;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int t = threadIdx.x, EY = pl.ey, EX = pl.ex, TY = EY - 1, TX = EX - 1;
+    const int PLN = ((EX + 1) * (EY + 1) * 3 * SZ + 15) / 16 * 16 / SZ;
+    // factor slots (16-byte pieces first), then the node planes
+    constexpr int WB = fine_stage_w<N, WT> ? N * N * N * (int)sizeof(WT) * TH : 0;
+    T *planes = reinterpret_cast<T *>(smem_raw + WB);            // 2 x PLN
+    T *corners = planes + 2 * PLN;                               // 2 x 9 x TH
+    T *sums = corners + 2 * 9 * TH;                              // 2 x 3 x TH, dense over the owned tile
+    double *epd = reinterpret_cast<double *>(sums + 2 * 3 * TH); // FINE_OUT: r, so; FINE_DOT: r (3 x TH each)
+    T *ept = MODE == FINE_OUT ? reinterpret_cast<T *>(epd + 6 * TH) : sums + 2 * 3 * TH;
+
+    const int by = blockIdx.x % pl.ty, bx = blockIdx.x / pl.ty % pl.tx, bz = blockIdx.x / (pl.ty * pl.tx);
+    const int y0 = by * TY, x0 = bx * TX, z0 = bz * pl.lz, z1 = min(z0 + pl.lz, g.nz);
+    const int64_t zs = (int64_t)3 * g.nx * g.ny;                 // values per node plane
+
+    // Staging: value f of the (EX + 1) x (EY + 1) x 3 halo of a plane, as its
+    // byte offset in the plane.  Values outside the mesh are never copied:
+    // their slots of both buffers are cleared here.
+    uint32_t goff[FINE_NQ];
+    {
+        const int rw = 3 * (EY + 1), n = (EX + 1) * rw;
+#pragma unroll
+        for (int q = 0; q < FINE_NQ; ++q) {
+            const int f = t + q * TH, row = f / rw, col = f - row * rw;
+            const int gx = x0 - 1 + row, gv = 3 * (y0 - 1) + col;
+            const bool in = f < n && gx >= 0 && gx < g.nx && gv >= 0 && gv < 3 * g.ny;
+            goff[q] = in ? (uint32_t)(gx * 3 * g.ny + gv) * SZ : FINE_NONE;
+            if (f < n && !in) planes[f] = planes[PLN + f] = T(0);
+        }
+    }
+    auto stage = [&](int p) {
+        T *dst = planes + (p & 1) * PLN + t;
+        const char *src = reinterpret_cast<const char *>(a.x + p * zs);
+#pragma unroll
+        for (int q = 0; q < FINE_NQ; ++q)
+            if (goff[q] != FINE_NONE) cp_async<SZ>(dst + q * TH, src + goff[q], true);
+    };
+    // output: value f of the TX x TY x 3 owned values of a plane
+    uint32_t ooff[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const int f = t + q * TH, row = f / (3 * TY), col = f - row * 3 * TY;
+        ooff[q] = row < TX && x0 + row < g.nx && 3 * y0 + col < 3 * g.ny
+                      ? (uint32_t)((x0 + row) * 3 * g.ny + 3 * y0 + col)
+                      : FINE_NONE;
+    }
+    // blocks without a fixed dof do not read the mask
+    const bool fixed = MASK && (!a.fixed || a.fixed[blockIdx.x]);
+
+    // this thread's element column and owned node
+    const int i = t / EY, j = t - i * EY, ex = x0 - 1 + i, ey = y0 - 1 + j;
+    const bool act = i < EX;
+    const bool inside = act && ex >= 0 && ex < g.nelx && ey >= 0 && ey < g.nely;
+    const bool own = act && i >= 1 && j >= 1;
+    const int ni = act ? (i * (EY + 1) + j) * 3 : 0;             // low corner in the staged plane
+    const int si = own ? ((i - 1) * TY + (j - 1)) * 3 : 0;       // node in the sums
+    const int64_t wrow = nely_d, wplane = (int64_t)nelx_d * nely_d;
+    const WT *wp = inside ? w + (int64_t)ex * N * wrow + ey * N : w;
+    unsigned char *wslot = smem_raw + t * FineSlot<N, WT>::BYTES;
+    auto stage_w = [&](int e) {
+        if (e >= 0 && e < g.nelz)
+            stage_factors<N, WT, TH>(wslot, wp + (inside ? (int64_t)e * N * wplane : 0), wrow, wplane, inside);
+    };
+
+    auto read_plane = [&](int p, PlaneModes<T> (&m)[3]) {
+        const T *s = planes + (p & 1) * PLN + ni;
+        const int up = act ? 3 * (EY + 1) : 0, hi = act ? 3 : 0;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) m[c] = plane_modes<T>(s[c], s[hi + c], s[up + c], s[up + hi + c]);
+    };
+
+    PlaneModes<T> lo[3];
+    T carry[3][4], ll[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        lo[c] = {T(0), T(0), T(0), T(0), T(0)};
+        ll[c] = T(0);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) carry[c][q] = T(0);
+    }
+    if (z0 > 0) stage(z0 - 1);
+    stage(z0);
+    stage_w(z0 - 1);
+    cp_async_commit();
+    cp_async_wait();
+    __syncthreads();
+    if (z0 > 0) read_plane(z0 - 1, lo);
+    __syncthreads();   // the slot of plane z0 - 1 is staged next
+
+    uint8_t mask[3] = {1, 1, 1};
+    double dot0 = 0.0, dot1 = 0.0;
+#pragma unroll UNROLL
+    for (int e = z0 - 1; e <= z1 + 1; ++e) {
+        // epilogue of plane e - 2
+        if (e - 2 >= z0) {
+            const T *sp = sums + (e & 1) * 3 * TH + t;
+            T *out = static_cast<T *>(a.out) + (e - 2) * zs;
+            double *out64 = static_cast<double *>(a.out) + (e - 2) * zs;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const uint32_t o = ooff[q];
+                if (o == FINE_NONE) continue;
+                const T v = sp[q * TH];
+                const T *et = ept + t + q * TH;
+                if constexpr (MODE == FINE_APPLY) {
+                    out[o] = mask[q] ? v : T(0);
+                } else if constexpr (MODE == FINE_DOT) {
+                    const T y = mask[q] ? v : T(0);
+                    out[o] = y;
+                    dot0 += epd[t + q * TH] * (double)y;
+                } else if constexpr (MODE == FINE_RESID) {
+                    out[o] = mask[q] ? et[0] - v : T(0);
+                } else if constexpr (MODE == FINE_JACOBI) {
+                    out[o] = et[2 * 3 * TH] + et[3 * TH] * (et[0] - v);
+                } else {
+                    const double *ed = epd + t + q * TH;
+                    const double r = ed[0], so = ed[3 * TH];
+                    const double s = (double)(et[3 * TH] + et[0] * ((T)r - v));
+                    out64[o] = s;
+                    dot0 += r * s;
+                    dot1 += r * so;
+                }
+            }
+        }
+        // inputs of the next layer, operands of plane e - 1
+        if (e + 2 <= z1 && e + 2 < g.nz) stage(e + 2);
+        if (e - 1 >= z0 && e - 1 < z1) {
+            const int64_t base = (e - 1) * zs;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const uint32_t o = ooff[q];
+                if (o == FINE_NONE) continue;
+                const int f = t + q * TH;
+                if (fixed) mask[q] = (a.fm + base)[o];
+                if constexpr (MODE == FINE_RESID) cp_async<SZ>(ept + f, (a.b + base) + o, true);
+                if constexpr (MODE == FINE_DOT) cp_async<8>(epd + f, (a.r + base) + o, true);
+                if constexpr (MODE == FINE_JACOBI) {
+                    cp_async<SZ>(ept + f, (a.b + base) + o, true);
+                    cp_async<SZ>(ept + 3 * TH + f, (a.invd + base) + o, true);
+                    cp_async<SZ>(ept + 2 * 3 * TH + f, (a.x + base) + o, true);
+                }
+                if constexpr (MODE == FINE_OUT) {
+                    cp_async<8>(epd + f, (a.r + base) + o, true);
+                    cp_async<8>(epd + 3 * TH + f, a.so ? (a.so + base) + o : a.r, a.so != nullptr);
+                    cp_async<SZ>(ept + f, (a.invd + base) + o, true);
+                    cp_async<SZ>(ept + 3 * TH + f, (a.x + base) + o, true);
+                }
+            }
+        }
+        const bool layer = e < z1 && e >= 0 && e < g.nelz;       // an element layer to compute
+        T wv[N * N * N];
+        if (layer)
+            load_factors<N, T, WT, TH>(wslot, wp + (inside ? (int64_t)e * N * wplane : 0), wrow, wplane, inside, wv);
+        if (e + 1 < z1) stage_w(e + 1);
+        cp_async_commit();
+
+        // node sums of plane e - 1: corners low-low of this column, x-high of
+        // column (i - 1, j), y-high of (i, j - 1) and high-high of (i - 1, j - 1)
+        if (e - 1 >= z0 && e - 1 < z1 && own) {
+            const T *cp = corners + ((e - 1) & 1) * 9 * TH;
+            T *sp = sums + ((e - 1) & 1) * 3 * TH + si;
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                sp[c] = ((ll[c] + cp[c * TH + t - EY]) + cp[(3 + c) * TH + t - 1]) + cp[(6 + c) * TH + t - EY - 1];
+        }
+
+        if (e < z1) {
+            PlaneModes<T> hi[3];
+            T top[3][4];
+            const bool corner = e >= z0;
+            T *cp = corners + (e & 1) * 9 * TH + t;
+            auto put = [&](int c, T c0, T cx, T cy, T cxy) {   // plane-e values of component c, as corners
+                const T p = c0 + cxy, q = cx + cy, p2 = c0 - cxy, q2 = cx - cy;
+                ll[c] = p - q;
+                cp[c * TH] = p2 + q2;
+                cp[(3 + c) * TH] = p2 - q2;
+                cp[(6 + c) * TH] = p + q;
+            };
+            if (e + 1 < g.nz) read_plane(e + 1, hi);
+            if (layer) {
+                T m[3][8], r[3][8], W[modal_moments<N>];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) element_modes<T>(lo[c], hi[c], m[c]);
+                modal_weights<N, T>(wv, W);
+                modal_stress<N, T>(m, W, k, r);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const T rxy = T(MODAL_R3) * r[c][3], rxz = T(MODAL_R3) * r[c][5], ryz = T(MODAL_R3) * r[c][6],
+                            rxyz = T(1.0 / 3.0) * r[c][7];
+                    if (corner)
+                        put(c, carry[c][0] - r[c][4], carry[c][1] + (r[c][1] - rxz), carry[c][2] + (r[c][2] - ryz),
+                            carry[c][3] + (rxy - rxyz));
+                    top[c][0] = r[c][4];
+                    top[c][1] = r[c][1] + rxz;
+                    top[c][2] = r[c][2] + ryz;
+                    top[c][3] = rxy + rxyz;
+                }
+            } else {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    if (corner) put(c, carry[c][0], carry[c][1], carry[c][2], carry[c][3]);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) top[c][q] = T(0);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                if (e + 1 < g.nz) lo[c] = hi[c];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) carry[c][q] = top[c][q];
+            }
+        }
+        cp_async_wait();
+        __syncthreads();
+    }
+
+    if constexpr (MODE == FINE_OUT || MODE == FINE_DOT) {
+        if (!a.o0) return;
+        double *sh = reinterpret_cast<double *>(smem_raw);
+        __shared__ bool last;
+        dot0 = fine_block_sum(dot0, sh);
+        if (MODE == FINE_OUT) dot1 = fine_block_sum(dot1, sh);
+        unsigned *counter = reinterpret_cast<unsigned *>(a.part + 2 * (int64_t)gridDim.x);
+        if (t == 0) {
+            a.part[blockIdx.x] = dot0;
+            a.part[gridDim.x + blockIdx.x] = dot1;
+            __threadfence();
+            last = atomicInc(counter, gridDim.x - 1) == gridDim.x - 1;
+        }
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+        double s0 = 0.0, s1 = 0.0;
+        for (unsigned b = t; b < gridDim.x; b += TH) {
+            s0 += __ldcg(a.part + b);
+            if (MODE == FINE_OUT) s1 += __ldcg(a.part + gridDim.x + b);
+        }
+        s0 = fine_block_sum(s0, sh);
+        if (MODE == FINE_OUT) s1 = fine_block_sum(s1, sh);
+        if (t == 0) {
+            *a.o0 = s0;
+            if (MODE == FINE_OUT && a.so) *a.o1 = s1;
+        }
+    }
+}
+
+ModalCoef<double> modal_coef(double el, double eh, double ew, double nu, int n) {
+    const double h[3] = {el, eh, ew};
+    const double lam = nu / ((1 + nu) * (1 - 2 * nu)), mu = 1 / (2 * (1 + nu));
+    // cell volume in local coordinates, element Jacobian, and the transforms' 1/8 twice
+    const double sc = 8.0 / (n * n * n) * (el * eh * ew / 8) / 64;
+    ModalCoef<double> k;
+    for (int c = 0; c < 3; ++c) {
+        k.t[c] = el / h[c];
+        k.kt[c] = lam * sc * (2 / el) * (2 / h[c]);
+        k.kn[c] = 2 * mu * sc * (2 / h[c]) * (2 / h[c]);
+    }
+    for (int q = 0; q < 3; ++q) {
+        const double hc = h[modal_sc(q)], hd = h[modal_sd(q)];
+        k.sr[q] = hd / hc;
+        k.s1[q] = mu * sc * (2 / hd) * (2 / hd);
+        k.s2[q] = mu * sc * (2 / hd) * (2 / hc);
+    }
+    return k;
+}
+
+// Tile and chunk of a mesh: the least modelled time over tile heights and
+// chunk counts.  An SM holds `res` blocks at a time; a layer of r resident
+// blocks takes r units, or the 1.6 units of a block's own latency, and a block
+// pays about three layers for its start and its drain besides the one below
+// its first plane.
+FinePlan fine_plan(const Grid &g, int n, int elem_bytes) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (sms < 1) sms = 148;
+    const int th = elem_bytes == 8 ? fine_threads<double> : fine_threads<float>;
+    const int res = fine_resident(n, elem_bytes);
+    auto layer = [](int r) { return r == 0 ? 0.0 : std::max((double)r, 1.6); };
+    FinePlan best;
+    double least = 1e300;
+    for (int ey = 2; ey <= 65 && ey <= g.ny + 1; ++ey) {
+        int ex = std::min(th / ey, g.nx + 1);
+        while (ex >= 2 && (ex + 1) * (ey + 1) * 3 > FINE_NQ * th) --ex;
+        if (ex < 2) continue;
+        const int ty = (g.ny + ey - 2) / (ey - 1), tx = (g.nx + ex - 2) / (ex - 1);
+        ex = (g.nx + tx - 1) / tx + 1;   // even tiles
+        const int64_t tiles = (int64_t)ty * tx;
+        for (int c = 1; c <= g.nz; ++c) {
+            const int lz = (g.nz + c - 1) / c, tz = (g.nz + lz - 1) / lz;
+            if (tz != c) continue;
+            const int64_t blocks = tiles * tz, per = (blocks + sms - 1) / sms;   // blocks of the busiest SM
+            const double cost = ((per / res) * layer(res) + layer(per % res)) * (lz + 4);
+            if (cost < least) {
+                least = cost;
+                best.ey = ey; best.ex = ex; best.lz = lz;
+                best.ty = ty; best.tx = tx; best.tz = tz;
+            }
+        }
+    }
+    return best;
+}
+
+// flag[b] = 1 when block b of the plan owns a node with a fixed dof.
+__global__ void k_fine_fixed(const uint8_t *__restrict__ fm, const Grid g, const FinePlan pl, uint8_t *flag) {
+    const int TY = pl.ey - 1, TX = pl.ex - 1;
+    const int by = blockIdx.x % pl.ty, bx = blockIdx.x / pl.ty % pl.tx, bz = blockIdx.x / (pl.ty * pl.tx);
+    const int y0 = by * TY, x0 = bx * TX, z0 = bz * pl.lz;
+    const int cy = min(TY, g.ny - y0), cx = min(TX, g.nx - x0), cz = min(pl.lz, g.nz - z0);
+    int any = 0;
+    for (int f = threadIdx.x; f < cz * cx * 3 * cy; f += blockDim.x) {
+        const int z = f / (cx * 3 * cy), x = f / (3 * cy) % cx, v = f % (3 * cy);
+        any |= !fm[3 * (((int64_t)(z0 + z) * g.nx + x0 + x) * g.ny + y0) + v];
+    }
+    any = __syncthreads_or(any);
+    if (threadIdx.x == 0) flag[blockIdx.x] = any ? 1 : 0;
+}
+
+void launch_fine_fixed(const uint8_t *fm, const Grid &g, const FinePlan &plan, uint8_t *flag, cudaStream_t st) {
+    k_fine_fixed<<<plan.blocks(), 256, 0, st>>>(fm, g, plan, flag);
+    count_launch();
+}
+
+template <int N, typename T, typename WT, int MODE>
+static void launch_mode(const FineArgs<T> &a, const WT *w, const FineGeom &fg, const FinePlan &plan,
+                        const ModalCoef<T> &k, cudaStream_t st) {
+    auto kern = k_fine_modal<N, T, WT, MODE>;
+    const size_t smem = fine_smem<N, T, WT, MODE>(plan);
+    if (smem > 47 * 1024)   // (the kernel has a few static bytes besides)
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kern<<<plan.blocks(), fine_threads<T>, smem, st>>>(a, w, fg.g, fg.nelx_d, fg.nely_d, plan, k);
+    count_launch();
+}
+
+template <int N, typename T, typename WT>
+static void launch_n(FineMode mode, const FineArgs<T> &a, const WT *w, const FineGeom &fg, const FinePlan &plan,
+                     const ModalCoef<T> &k, cudaStream_t st) {
+    switch (mode) {
+        case FINE_APPLY: return launch_mode<N, T, WT, FINE_APPLY>(a, w, fg, plan, k, st);
+        case FINE_RESID: return launch_mode<N, T, WT, FINE_RESID>(a, w, fg, plan, k, st);
+        case FINE_JACOBI: return launch_mode<N, T, WT, FINE_JACOBI>(a, w, fg, plan, k, st);
+        case FINE_OUT: return launch_mode<N, T, WT, FINE_OUT>(a, w, fg, plan, k, st);
+        case FINE_DOT: return launch_mode<N, T, WT, FINE_DOT>(a, w, fg, plan, k, st);
+    }
+}
+
+template <typename T, typename WT>
+void launch_fine_modal(int n, FineMode mode, const FineArgs<T> &a, const WT *w, const FineGeom &fg,
+                       const FinePlan &plan, const ModalCoef<T> &k, cudaStream_t st) {
+    if (n == 1) launch_n<1, T, WT>(mode, a, w, fg, plan, k, st);
+    else if (n == 2) launch_n<2, T, WT>(mode, a, w, fg, plan, k, st);
+    else launch_n<3, T, WT>(mode, a, w, fg, plan, k, st);
+}
+
+template void launch_fine_modal<double, double>(int, FineMode, const FineArgs<double> &, const double *,
+                                                const FineGeom &, const FinePlan &, const ModalCoef<double> &,
+                                                cudaStream_t);
+template void launch_fine_modal<float, float>(int, FineMode, const FineArgs<float> &, const float *,
+                                              const FineGeom &, const FinePlan &, const ModalCoef<float> &,
+                                              cudaStream_t);
+template void launch_fine_modal<float, __nv_bfloat16>(int, FineMode, const FineArgs<float> &, const __nv_bfloat16 *,
+                                                      const FineGeom &, const FinePlan &, const ModalCoef<float> &,
+                                                      cudaStream_t);
+
+}  // namespace tosp

@@ -105,16 +105,14 @@ __device__ __forceinline__ double sum_partials(const double *partials, int np, d
     return block_sum(s, sh);
 }
 
-template <typename TB>
-__global__ void __launch_bounds__(256, 4) k_dot_partial(const double *a, const TB *b, int64_t n, double *partials, double *out) {
+__global__ void __launch_bounds__(256, 4) k_dot_partial(const double *a, const double *b, int64_t n, double *partials, double *out) {
     __shared__ double sh[32];
     double s = 0.0;
     constexpr int VB8 = 2 * VB;
-    double av[VB8];
-    TB bv[VB8];
+    double av[VB8], bv[VB8];
     grid_batched<VB8>(
         n, [&](int k, int64_t i) { av[k] = a[i]; bv[k] = b[i]; },
-        [&](int k, int64_t) { s += av[k] * (double)bv[k]; });
+        [&](int k, int64_t) { s += av[k] * bv[k]; });
     s = block_sum(s, sh);
     if (threadIdx.x == 0) partials[blockIdx.x] = s;
     if (last_block(red_counter(partials))) {
@@ -124,10 +122,7 @@ __global__ void __launch_bounds__(256, 4) k_dot_partial(const double *a, const T
 }
 
 void launch_dot(const double *a, const double *b, int64_t n, double *partials, double *out, cudaStream_t st) {
-    k_dot_partial<double><<<RED_BLOCKS, 256, 0, st>>>(a, b, n, partials, out); count_launch();
-}
-void launch_dot(const double *a, const float *b, int64_t n, double *partials, double *out, cudaStream_t st) {
-    k_dot_partial<float><<<RED_BLOCKS, 256, 0, st>>>(a, b, n, partials, out); count_launch();
+    k_dot_partial<<<RED_BLOCKS, 256, 0, st>>>(a, b, n, partials, out); count_launch();
 }
 
 // a'b and a'c in one pass over a (partials: 2 * RED_BLOCKS).
@@ -163,63 +158,6 @@ void launch_dot2(const double *a, const double *b, const double *c, int64_t n, d
     k_dot2_partial<<<RED_BLOCKS, 256, 0, st>>>(a, b, c, n, partials, out0, out1); count_launch();
 }
 
-// The finest post-sweep of the preconditioner written as the FP64 CG vector,
-// s = x + invd (b - t) (k_jacobi_out), with the CG's dots of the new s in the
-// same pass: r's -> out0 and, when so is given, r's_old -> out1.  Same grid,
-// loop order and reduction tree as k_dot2_partial / k_dot_partial, so the
-// dots are bitwise those of the separate kernels.
-template <typename T>
-__global__ void __launch_bounds__(256, 4) k_jacobi_out_dot(double *out, const T *x, const T *b, const T *t, const T *invd, int64_t n,
-                                 const double *r, const double *so, double *partials, double *out0, double *out1) {
-    __shared__ double sh[32];
-    double s0 = 0.0, s1 = 0.0;
-    T xv[VB], bv[VB], tv[VB], dv[VB];
-    double rv[VB], ov[VB];
-    grid_batched(
-        n,
-        [&](int k, int64_t i) {
-            xv[k] = x[i];
-            bv[k] = b[i];
-            tv[k] = t[i];
-            dv[k] = invd[i];
-            rv[k] = r[i];
-            if (so) ov[k] = so[i];
-        },
-        [&](int k, int64_t i) {
-            const double si = (double)(xv[k] + dv[k] * (bv[k] - tv[k]));
-            out[i] = si;
-            s0 += rv[k] * si;
-            if (so) s1 += rv[k] * ov[k];
-        });
-    s0 = block_sum(s0, sh);
-    if (so) s1 = block_sum(s1, sh);
-    if (threadIdx.x == 0) {
-        partials[blockIdx.x] = s0;
-        partials[RED_BLOCKS + blockIdx.x] = s1;
-    }
-    if (last_block(red_counter(partials))) {
-        const double t0 = sum_partials(partials, gridDim.x, sh);
-        const double t1 = so ? sum_partials(partials + RED_BLOCKS, gridDim.x, sh) : 0.0;
-        if (threadIdx.x == 0) {
-            out0[0] = t0;
-            if (so) out1[0] = t1;
-        }
-    }
-}
-
-template <typename T>
-void launch_jacobi_out_dot(double *out, const T *x, const T *b, const T *t, const T *invd, int64_t n, const double *r,
-                           const double *so, double *partials, double *out0, double *out1, cudaStream_t st) {
-    k_jacobi_out_dot<T><<<RED_BLOCKS, 256, 0, st>>>(out, x, b, t, invd, n, r, so, partials, out0, out1);
-    count_launch();
-}
-template void launch_jacobi_out_dot<float>(double *, const float *, const float *, const float *, const float *,
-                                           int64_t, const double *, const double *, double *, double *, double *,
-                                           cudaStream_t);
-template void launch_jacobi_out_dot<double>(double *, const double *, const double *, const double *, const double *,
-                                            int64_t, const double *, const double *, double *, double *, double *,
-                                            cudaStream_t);
-
 // Scalar slots (see solver.cpp): 0 rho, 1 gamma2 (previous rho), 2 d'q, 3 r'r,
 // 5 r's_old, 6 the previous iteration's alpha.  mode 1: first iteration
 // (d = s); 0: beta = rho/gamma2 (I/SolveMG.m:43-46); 2: flexible beta =
@@ -227,8 +165,7 @@ template void launch_jacobi_out_dot<double>(double *, const double *, const doub
 // iteration's s_old).  The iterate update of the previous iteration,
 // x += alpha d (I/SolveMG.m:40), is done here, while d is read anyway, before
 // d is replaced (modes 0 and 2); launch_pcg_finish applies the last one.
-// d32 (optional) receives the new d in FP32, the input of the tensor-core
-// product.
+// d32 (optional) receives the new d in FP32, the input of the FP32 product.
 __global__ void k_pcg_direction(double *d, const double *s, double *sold, const double *scal, int64_t n, int mode,
                                 double *x, float *d32) {
     const double beta = mode == 1 ? 0.0 : (mode == 2 ? (scal[0] - scal[5]) / scal[1] : scal[0] / scal[1]);

@@ -52,21 +52,20 @@ struct tosp_handle {
     Grid dens{};               // density (= design) mesh as a grid of elements
     int64_t nfree = 0;
     int64_t *d_freeidx = nullptr;
-    uint8_t *d_bfix = nullptr;      // per finest brick: touches a fixed dof
     // constants
     double *d_ke64 = nullptr;       // blocks packed per s (coarse build, Grad)
     double *d_cbS = nullptr;        // sub-cell Galerkin table of the finest coarsening
-    double *d_kt64 = nullptr;       // pair-major layout of the fine operator
-    float *d_kt32 = nullptr;
-    std::vector<double> ktab_c;     // MR 2: FP64 Walsh-Hadamard coefficients passed with each launch
-    uint16_t *d_tcimg = nullptr;    // mixed: tensor-core B operand image of the blocks (null: CUDA-core kernel)
-    int *d_tcerr = nullptr;         // set by the tensor-core operator when an MMA wait times out
-    uint16_t *d_tcimg32 = nullptr;  // cg_product 1: B image of the CG's product (three-piece blocks)
+    // finest operator: constants of the modal product, tile plan
+    ModalCoef<double> mk64{};
+    ModalCoef<float> mk32{};
+    FinePlan plan64, plan32;
+    uint8_t *d_fix64 = nullptr, *d_fix32 = nullptr;   // per block of the plans: owns a fixed dof
+    double *d_part64 = nullptr, *d_part32 = nullptr;  // the plans' partial dots and arrival counter
     // densities
     double *d_rho = nullptr, *d_w64 = nullptr;
     double *d_wq = nullptr;         // mixed: BF16-rounded factors in FP64 (V-cycle hierarchy)
     __nv_bfloat16 *d_wbf = nullptr;
-    float *d_w32 = nullptr;         // cg_product 1: FP32 factors of the CG's tensor-core product
+    float *d_w32 = nullptr;         // cg_product 1: FP32 factors of the CG's FP32 product
     uint8_t *d_free_elem = nullptr;
     // filter
     FilterTap *d_taps = nullptr;
@@ -90,7 +89,8 @@ struct tosp_handle {
     // and three step lists (entered with the first sweep done, from zero, warm)
     // dots the CG wants from the preconditioner's last sweep (cg_iteration)
     struct {
-        const double *r = nullptr, *so = nullptr;
+        const double *rhs = nullptr;   // the cycle's FP64 right-hand side
+        const double *so = nullptr;
         double *o0 = nullptr, *o1 = nullptr;
         bool want = false, done = false;
     } fdot;
@@ -106,7 +106,7 @@ struct tosp_handle {
     bool graph_failed = false;
     // CG (FP64, full-length vectors with zeros on fixed dofs)
     double *cx = nullptr, *cr = nullptr, *cd = nullptr, *cq = nullptr, *cs = nullptr, *cf = nullptr, *cso = nullptr;
-    // cg_product 1: the direction in FP32 and its tensor-core product
+    // cg_product 1: the direction in FP32 and its product
     bool cg32 = false;
     float *cd32 = nullptr, *cq32 = nullptr;
     double *d_partials = nullptr, *d_scal = nullptr, *h_scal = nullptr;
@@ -247,43 +247,43 @@ int choose_levels(int nelx, int nely, int nelz, int ngrids, int nmaxchol, int op
 }
 
 // ----- operators -------------------------------------------------------------
-// The FP64 finest-level kernel (coefficients as a launch parameter for MR 2).
-void launch_fine64(tosp_handle *h, const double *x, double *y) {
-    if (h->n == 2 && !h->ktab_c.empty())
-        launch_fine_apply64_const(x, y, h->d_w64, h->lev[0].fm, h->ktab_c.data(), h->fg, h->stream);
+// A product of the finest operator with FP64 factors (T double), with the
+// V-cycle's BF16 factors (T float), or the CG's FP32 factors (cg32).
+template <typename T>
+void launch_fine(tosp_handle *h, FineMode mode, const FineArgs<T> &args, bool cg32 = false) {
+    FineArgs<T> a = args;
+    a.fm = h->lev[0].fm;
+    a.fixed = sizeof(T) == 8 ? h->d_fix64 : h->d_fix32;
+    a.part = sizeof(T) == 8 ? h->d_part64 : h->d_part32;
+    if constexpr (sizeof(T) == 8)
+        launch_fine_modal<double, double>(h->n, mode, a, h->d_w64, h->fg, h->plan64, h->mk64, h->stream);
+    else if (cg32)
+        launch_fine_modal<float, float>(h->n, mode, a, h->d_w32, h->fg, h->plan32, h->mk32, h->stream);
     else
-        launch_fine_apply<double, double>(x, y, h->d_w64, h->lev[0].fm, h->d_kt64, h->fg, h->n, h->stream);
+        launch_fine_modal<float, __nv_bfloat16>(h->n, mode, a, h->d_wbf, h->fg, h->plan32, h->mk32, h->stream);
 }
 
-// y = K x at the finest level in the cycle precision (zeroes y first).
+// y = K x at the finest level (every dof of y is written).
 template <typename T>
-int fine_apply(tosp_handle *h, const T *x, T *y) {
-    CK(cudaMemsetAsync(y, 0, sizeof(T) * h->fg.g.ndof, h->stream));
-    if constexpr (sizeof(T) == 8) {
-        launch_fine64(h, x, y);
-    } else if (h->d_tcimg) {
-        launch_fine_apply_tc(x, y, h->d_wbf, h->lev[0].fm, h->d_tcimg, h->fg, h->n, h->d_tcerr, h->stream);
-    } else {
-        launch_fine_apply<float, __nv_bfloat16>(x, y, h->d_wbf, h->lev[0].fm, h->d_kt32, h->fg, h->n, h->stream);
-    }
+int fine_apply(tosp_handle *h, const T *x, T *y, bool cg32 = false) {
+    FineArgs<T> a;
+    a.x = x;
+    a.out = y;
+    launch_fine<T>(h, FINE_APPLY, a, cg32);
     CKL();
     return TOSP_OK;
 }
 
 int fine_apply64(tosp_handle *h, const double *x, double *y) { return fine_apply<double>(h, x, y); }
 
-// cg_product 1: the CG's product y = K x on the tensor cores with FP32 factors.
-int fine_apply_cg32(tosp_handle *h, const float *x, float *y) {
-    CK(cudaMemsetAsync(y, 0, sizeof(float) * h->fg.g.ndof, h->stream));
-    launch_fine_apply_tc_w32(x, y, h->d_w32, h->lev[0].fm, h->d_tcimg32, h->fg, h->n, h->d_tcerr, h->stream);
-    CKL();
-    return TOSP_OK;
-}
+// cg_product 1: the CG's product y = K x in FP32.
+int fine_apply_cg32(tosp_handle *h, const float *x, float *y) { return fine_apply<float>(h, x, y, true); }
 
 // Damped Jacobi sweeps (I/Smooth.m:14-23).  first_done: the first sweep from
 // a zero guess was already written into lev[l].x (fused into the CG update);
 // out (finest level only): the last sweep is written to out in FP64 instead of
-// lev[l].x (the preconditioned vector of the outer CG).
+// lev[l].x (the preconditioned vector of the outer CG).  A sweep is one launch:
+// the product's kernel updates the iterate where it has K x.
 template <typename T>
 int smooth(tosp_handle *h, int l, int niter, bool x_zero, bool first_done = false, double *out = nullptr) {
     Level &L = h->lev[l];
@@ -293,17 +293,27 @@ int smooth(tosp_handle *h, int l, int niter, bool x_zero, bool first_done = fals
     for (int it = 0; it < niter; ++it) {
         const bool first = x_zero && it == 0;
         if (first) {
-            if (!first_done) launch_jacobi_update<T>((T *)L.x, b, nullptr, (const T *)L.invd, nd, 1, h->stream);
+            if (!first_done) launch_jacobi_zero<T>((T *)L.x, b, (const T *)L.invd, nd, h->stream);
         } else if (l == 0) {
-            TRY(fine_apply<T>(h, (const T *)L.x, (T *)L.t));
-            if (out && it == niter - 1 && h->fdot.want) {
-                launch_jacobi_out_dot<T>(out, (const T *)L.x, b, (const T *)L.t, (const T *)L.invd, nd, h->fdot.r,
-                                         h->fdot.so, h->d_partials, h->fdot.o0, h->fdot.o1, h->stream);
-                h->fdot.done = true;
-            } else if (out && it == niter - 1)
-                launch_jacobi_out<T>(out, (const T *)L.x, b, (const T *)L.t, (const T *)L.invd, nd, h->stream);
-            else
-                launch_jacobi_update<T>((T *)L.x, b, (const T *)L.t, (const T *)L.invd, nd, 0, h->stream);
+            FineArgs<T> a;
+            a.x = (const T *)L.x;
+            a.invd = (const T *)L.invd;
+            if (out && it == niter - 1) {
+                a.out = out;
+                a.r = h->fdot.rhs;
+                if (h->fdot.want) {
+                    a.so = h->fdot.so;
+                    a.o0 = h->fdot.o0;
+                    a.o1 = h->fdot.o1;
+                    h->fdot.done = true;
+                }
+                launch_fine<T>(h, FINE_OUT, a);
+            } else {
+                a.out = L.t;
+                a.b = b;
+                launch_fine<T>(h, FINE_JACOBI, a);
+                std::swap(L.x, L.t);
+            }
         } else {
             launch_stencil<T>((const T *)L.st, (const T *)L.x, b, (const T *)L.invd, (T *)L.t, L.g, 2, L.nm,
                               h->stream);
@@ -318,8 +328,11 @@ template <typename T>
 int residual(tosp_handle *h, int l) {
     Level &L = h->lev[l];
     if (l == 0) {
-        TRY(fine_apply<T>(h, (const T *)L.x, (T *)L.t));
-        launch_residual<T>((const T *)L.b, (const T *)L.t, (T *)L.r, L.g.ndof, h->stream);
+        FineArgs<T> a;
+        a.x = (const T *)L.x;
+        a.b = (const T *)L.b;
+        a.out = L.r;
+        launch_fine<T>(h, FINE_RESID, a);
     } else {
         launch_stencil<T>((const T *)L.st, (const T *)L.x, (const T *)L.b, nullptr, (T *)L.r, L.g, 1, L.nm,
                           h->stream);
@@ -531,14 +544,8 @@ int cycle_vw(tosp_handle *h, int l, bool x_zero, bool wcycle, bool first_done = 
     const bool fuse = l + 1 < Lc && h->mg.smoothiter1 >= 1;
     const T *cinvd = fuse ? (const T *)C.invd : nullptr;
     T *cx = fuse ? (T *)C.x : nullptr;
-    if (l == 0) {
-        // finest residual b - A x restricted directly (no residual vector)
-        TRY(fine_apply<T>(h, (const T *)L.x, (T *)L.t));
-        launch_restrict_res<T>((const T *)L.b, (const T *)L.t, (T *)C.b, C.fm, L.g, C.g, h->stream, cinvd, cx);
-    } else {
-        TRY(residual<T>(h, l));
-        launch_restrict<T>((const T *)L.r, (T *)C.b, C.fm, L.g, C.g, h->stream, cinvd, cx);
-    }
+    TRY(residual<T>(h, l));
+    launch_restrict<T>((const T *)L.r, (T *)C.b, C.fm, L.g, C.g, h->stream, cinvd, cx);
     CKL();
     if (l + 1 == Lc) {
         TRY(coarse_solve<T>(h));
@@ -581,6 +588,10 @@ int precondition(tosp_handle *h, const double *r, double *s, bool prepared = fal
     Level &F = h->lev[0];
     const int64_t nd = F.g.ndof;
     double *out = h->mg.smoothiter2 >= 1 ? s : nullptr;
+    h->fdot.rhs = r;
+    // sweeps on the finest level swap its x and t; both are put back at the end,
+    // so that a captured iteration finds the buffers it was captured with
+    void *const x0 = F.x, *const t0 = F.t;
     if (h->precision == TOSP_PREC_FP64) {
         // the finest level reads r in place
         void *own_b = F.b;
@@ -588,7 +599,11 @@ int precondition(tosp_handle *h, const double *r, double *s, bool prepared = fal
         int rc = h->mg.cycle == 2 ? cycle_fmv<double>(h, 0, out) : cycle_vw<double>(h, 0, true, h->mg.cycle == 1,
                                                                                      false, out);
         F.b = own_b;
-        TRY(rc);
+        if (rc != TOSP_OK) {
+            F.x = x0;
+            F.t = t0;
+            return rc;
+        }
         if (!out) CK(cudaMemcpyAsync(s, F.x, sizeof(double) * nd, cudaMemcpyDeviceToDevice, h->stream));
     } else {
         if (!prepared) {
@@ -596,13 +611,20 @@ int precondition(tosp_handle *h, const double *r, double *s, bool prepared = fal
             CKL();
         }
         const bool first_done = prepared && fused_first_sweep(h);
-        if (h->mg.cycle == 2) TRY(cycle_fmv<float>(h, 0, out));
-        else TRY(cycle_vw<float>(h, 0, true, h->mg.cycle == 1, first_done, out));
+        const int rc = h->mg.cycle == 2 ? cycle_fmv<float>(h, 0, out)
+                                        : cycle_vw<float>(h, 0, true, h->mg.cycle == 1, first_done, out);
+        if (rc != TOSP_OK) {
+            F.x = x0;
+            F.t = t0;
+            return rc;
+        }
         if (!out) {
             launch_convert<float, double>((const float *)F.x, s, nd, h->stream);
             CKL();
         }
     }
+    F.x = x0;
+    F.t = t0;
     return TOSP_OK;
 }
 
@@ -668,25 +690,13 @@ int build_masks(tosp_handle *h, const int64_t *freedofs, int64_t nfree) {
     h->nfree = nfree;
     CK(cudaMemcpy(h->d_freeidx, idx.data(), sizeof(int64_t) * nfree, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(h->lev[0].fm, fm.data(), g0.ndof, cudaMemcpyHostToDevice));
-    // bricks whose nodes carry a fixed dof: a node at x lies in brick x / BX
-    // and, on a brick boundary, in brick x / BX - 1 (same in y and z)
-    {
-        const FineGeom &fg = h->fg;
-        std::vector<uint8_t> bf((size_t)fg.nbricks, 0);
-        for (int64_t d = 0; d < g0.ndof; ++d) {
-            if (fm[d]) continue;
-            const int64_t node = d / 3;
-            const int ny = (int)(node % g0.ny), nx = (int)((node / g0.ny) % g0.nx), nz = (int)(node / ((int64_t)g0.ny * g0.nx));
-            for (int bz = (nz - 1) / BZ; bz <= nz / BZ; ++bz)
-                for (int bx = (nx - 1) / BX; bx <= nx / BX; ++bx)
-                    for (int by = (ny - 1) / BY; by <= ny / BY; ++by)
-                        if (bx >= 0 && by >= 0 && bz >= 0 && bx < fg.nbx && by < fg.nby && bz < fg.nbz)
-                            bf[((size_t)bz * fg.nbx + bx) * fg.nby + by] = 1;
-        }
-        if (h->d_bfix == nullptr) TRY(dalloc(h, &h->d_bfix, fg.nbricks));
-        CK(cudaMemcpy(h->d_bfix, bf.data(), bf.size(), cudaMemcpyHostToDevice));
-        h->fg.bfix = h->d_bfix;
+    if (!h->d_fix64) TRY(dalloc(h, &h->d_fix64, h->plan64.blocks()));
+    launch_fine_fixed(h->lev[0].fm, g0, h->plan64, h->d_fix64, h->stream);
+    if (h->precision == TOSP_PREC_MIXED) {
+        if (!h->d_fix32) TRY(dalloc(h, &h->d_fix32, h->plan32.blocks()));
+        launch_fine_fixed(h->lev[0].fm, g0, h->plan32, h->d_fix32, h->stream);
     }
+    CKL();
     for (int l = 0; l + 1 < h->ngrids; ++l)
         launch_coarse_freemask(h->lev[l].fm, h->lev[l + 1].fm, h->lev[l].g, h->lev[l + 1].g, h->stream);
     CKL();
@@ -724,9 +734,8 @@ int create_impl(tosp_handle *h, const tosp_problem *pb, const tosp_mg_params *mg
         h->err = "cg_product must be 0 or 1 and replace_drop in [0, 1)";
         return TOSP_ERR_BAD_ARG;
     }
-    if (mg->cg_product == 1 && (precision != TOSP_PREC_MIXED || !fine_tc_supported(pb->mr_n, pb->nely) ||
-                                !fine_tc_w32_supported(pb->mr_n))) {
-        h->err = "cg_product 1 needs TOSP_PREC_MIXED and the tensor-core operator (n * nely even)";
+    if (mg->cg_product == 1 && (precision != TOSP_PREC_MIXED || pb->mr_n * pb->nely % 2 != 0)) {
+        h->err = "cg_product 1 needs TOSP_PREC_MIXED and n * nely even";
         return TOSP_ERR_UNSUPPORTED;
     }
     if (!pb->freedofs || pb->nfree <= 0) {
@@ -768,10 +777,6 @@ int create_impl(tosp_handle *h, const tosp_problem *pb, const tosp_mg_params *mg
     fg.g = g0;
     fg.nelx_d = pb->nelx * h->n;
     fg.nely_d = pb->nely * h->n;
-    fg.nbx = (g0.nelx + BX - 1) / BX;
-    fg.nby = (g0.nely + BY - 1) / BY;
-    fg.nbz = (g0.nelz + BZ - 1) / BZ;
-    fg.nbricks = (int64_t)fg.nbx * fg.nby * fg.nbz;
     h->dens = make_grid(pb->nelx * h->n, pb->nely * h->n, pb->nelz * h->n);
     h->ncoarse = h->mg_ok ? h->lev[ng - 1].g.ndof : 0;
     h->coarse_pcg = h->mg_ok && cpcg;
@@ -795,28 +800,18 @@ int create_impl(tosp_handle *h, const tosp_problem *pb, const tosp_mg_params *mg
         CK(cudaMemcpy(h->d_cbS, S.data(), sizeof(double) * S.size(), cudaMemcpyHostToDevice));
     }
     {
-        std::vector<double> kt64, kt32d;
-        fine_block_table(packed, h->n, 8, kt64);
-        if (h->n == 2) fine_mr2_const_table(kt64, 8, h->ktab_c);
-        fine_block_table(packed, h->n, 4, kt32d);
-        std::vector<float> kt32(kt32d.begin(), kt32d.end());
-        TRY(dalloc(h, &h->d_kt64, (int64_t)kt64.size()));
-        TRY(dalloc(h, &h->d_kt32, (int64_t)kt32.size()));
-        CK(cudaMemcpy(h->d_kt64, kt64.data(), sizeof(double) * kt64.size(), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(h->d_kt32, kt32.data(), sizeof(float) * kt32.size(), cudaMemcpyHostToDevice));
-    }
-    if (precision == TOSP_PREC_MIXED && fine_tc_supported(h->n, pb->nely)) {
-        std::vector<uint16_t> img;
-        fine_tc_image(packed, h->n, img);
-        TRY(dalloc(h, &h->d_tcimg, (int64_t)img.size()));
-        CK(cudaMemcpy(h->d_tcimg, img.data(), sizeof(uint16_t) * img.size(), cudaMemcpyHostToDevice));
-        TRY(dalloc(h, &h->d_tcerr, 1));
-        CK(cudaMemset(h->d_tcerr, 0, sizeof(int)));
-        if (mg->cg_product == 1) {
-            fine_tc_image_w32(packed, h->n, img);
-            TRY(dalloc(h, &h->d_tcimg32, (int64_t)img.size()));
-            CK(cudaMemcpy(h->d_tcimg32, img.data(), sizeof(uint16_t) * img.size(), cudaMemcpyHostToDevice));
+        const ModalCoef<double> k = modal_coef(pb->el, pb->eh, pb->ew, pb->nu, h->n);
+        h->mk64 = k;
+        for (int c = 0; c < 3; ++c) {
+            h->mk32.t[c] = (float)k.t[c];
+            h->mk32.kt[c] = (float)k.kt[c];
+            h->mk32.kn[c] = (float)k.kn[c];
+            h->mk32.sr[c] = (float)k.sr[c];
+            h->mk32.s1[c] = (float)k.s1[c];
+            h->mk32.s2[c] = (float)k.s2[c];
         }
+        h->plan64 = fine_plan(g0, h->n, 8);
+        h->plan32 = fine_plan(g0, h->n, 4);
     }
 
     // levels
@@ -901,6 +896,12 @@ int create_impl(tosp_handle *h, const tosp_problem *pb, const tosp_mg_params *mg
     }
     TRY(dalloc(h, &h->d_partials, 2 * RED_BLOCKS + 1));   // + the reductions' arrival counter
     CK(cudaMemset(h->d_partials, 0, sizeof(double) * (2 * RED_BLOCKS + 1)));
+    TRY(dalloc(h, &h->d_part64, 2 * (int64_t)h->plan64.blocks() + 1));
+    CK(cudaMemset(h->d_part64, 0, sizeof(double) * (2 * (int64_t)h->plan64.blocks() + 1)));
+    if (precision == TOSP_PREC_MIXED) {
+        TRY(dalloc(h, &h->d_part32, 2 * (int64_t)h->plan32.blocks() + 1));
+        CK(cudaMemset(h->d_part32, 0, sizeof(double) * (2 * (int64_t)h->plan32.blocks() + 1)));
+    }
     TRY(dalloc(h, &h->d_scal, 16));
     CK(cudaMallocHost(&h->h_scal, sizeof(double) * 16));
     TRY(dalloc(h, &h->d_ufull, g0.ndof));
@@ -1013,9 +1014,9 @@ int need_mg(tosp_handle *h) {
     return TOSP_OK;
 }
 
-// Reads (and clears) the tensor-core operator's timeout flag; call after a
-// stream synchronisation.
-int check_tc(tosp_handle *h) {
+// Reads (and clears) the timeout flags of the cooperative kernels' bounded
+// waits; call after a stream synchronisation.
+int check_waits(tosp_handle *h) {
     if (h->cpw.bar) {
         GridBarrier b{};
         CK(cudaMemcpy(&b, h->cpw.bar, sizeof b, cudaMemcpyDeviceToHost));
@@ -1033,15 +1034,6 @@ int check_tc(tosp_handle *h) {
             h->err = "persistent coarse cycle: grid barrier wait timed out";
             return TOSP_ERR_TIMEOUT;
         }
-    }
-    if (!h->d_tcerr) return TOSP_OK;
-    int e = 0;
-    CK(cudaMemcpy(&e, h->d_tcerr, sizeof(int), cudaMemcpyDeviceToHost));
-    if (e) {
-        CK(cudaMemset(h->d_tcerr, 0, sizeof(int)));
-        h->err = e == 2 ? "tensor-core operator: dynamic shared memory not 16-byte aligned"
-                        : "tensor-core operator: wait for MMA completion timed out";
-        return TOSP_ERR_TIMEOUT;
     }
     return TOSP_OK;
 }
@@ -1075,7 +1067,6 @@ int cg_iteration(tosp_handle *h, int mode, int k) {
     // previous update (mixed precision)
     // the dots of the new s ride on the preconditioner's last sweep when it
     // writes s (post-smoothing), else they take their own pass
-    h->fdot.r = h->cr;
     h->fdot.so = mode == 2 ? s_old : nullptr;
     h->fdot.o0 = h->d_scal + 0;
     h->fdot.o1 = h->d_scal + 5;
@@ -1095,12 +1086,20 @@ int cg_iteration(tosp_handle *h, int mode, int k) {
     const float *invd0 = first ? (const float *)F.invd : nullptr;
     float *x0 = first ? (float *)F.x : nullptr;
     if (h->cg32) {
-        TRY(fine_apply_cg32(h, h->cd32, h->cq32));
-        launch_dot(h->cd, (const float *)h->cq32, nd, h->d_partials, h->d_scal + 2, h->stream);
+        FineArgs<float> a;
+        a.x = h->cd32;
+        a.out = h->cq32;
+        a.r = h->cd;
+        a.o0 = h->d_scal + 2;
+        launch_fine<float>(h, FINE_DOT, a, true);
         launch_pcg_update(h->cr, (const float *)h->cq32, h->d_scal, h->d_partials, nd, h->stream, b0, invd0, x0);
     } else {
-        TRY(fine_apply64(h, h->cd, h->cq));
-        launch_dot(h->cd, h->cq, nd, h->d_partials, h->d_scal + 2, h->stream);
+        FineArgs<double> a;
+        a.x = h->cd;
+        a.out = h->cq;
+        a.r = h->cd;
+        a.o0 = h->d_scal + 2;
+        launch_fine<double>(h, FINE_DOT, a);
         launch_pcg_update(h->cr, h->cq, h->d_scal, h->d_partials, nd, h->stream, b0, invd0, x0);
     }
     CKL();
@@ -1139,8 +1138,11 @@ int solve_init(tosp_handle *h) {
     if (h->h_scal[3] == 0.0) {
         CK(cudaMemcpyAsync(h->cr, h->cf, sizeof(double) * nd, cudaMemcpyDeviceToDevice, h->stream));
     } else {
-        TRY(fine_apply64(h, h->cx, h->cq));
-        launch_residual<double>(h->cf, h->cq, h->cr, nd, h->stream);
+        FineArgs<double> a;
+        a.x = h->cx;
+        a.b = h->cf;
+        a.out = h->cr;
+        launch_fine<double>(h, FINE_RESID, a);
         CKL();
     }
     launch_dot(h->cf, h->cf, nd, h->d_partials, h->d_scal + 4, h->stream);
@@ -1221,7 +1223,7 @@ int solve_finish(tosp_handle *h, int32_t *it_out, double *relres_out) {
     h->stats.it = S.it;
     h->stats.relres = S.nr;
     h->stats.replacements = S.replaced;
-    TRY(check_tc(h));
+    TRY(check_waits(h));
     return S.rc;
 }
 
@@ -1637,7 +1639,7 @@ int tosp_kelem_prod_mixed(tosp_handle *h, const double *x, double *y, int64_t nf
     CKL();
     TRY(full_to_free(h, h->cq, y, "y"));
     TRY(sync(h));
-    return check_tc(h);
+    return check_waits(h);
 }
 
 int tosp_kelem_prod_cg32(tosp_handle *h, const double *x, double *y, int64_t nfree) {
@@ -1645,7 +1647,7 @@ int tosp_kelem_prod_cg32(tosp_handle *h, const double *x, double *y, int64_t nfr
     if (!h || !x || !y) return TOSP_ERR_BAD_ARG;
     cudaSetDevice(h->device);
     if (!h->cg32) {
-        h->err = "the CG's tensor-core product exists only on handles created with cg_product 1";
+        h->err = "the CG's FP32 product exists only on handles created with cg_product 1";
         return TOSP_ERR_STATE;
     }
     TRY(check_len(h, nfree, h->nfree, "x"));
@@ -1659,7 +1661,7 @@ int tosp_kelem_prod_cg32(tosp_handle *h, const double *x, double *y, int64_t nfr
     CKL();
     TRY(full_to_free(h, h->cq, y, "y"));
     TRY(sync(h));
-    return check_tc(h);
+    return check_waits(h);
 }
 
 int tosp_mg_cycle(tosp_handle *h, const double *r, double *s, int64_t nfree) {
@@ -1673,7 +1675,7 @@ int tosp_mg_cycle(tosp_handle *h, const double *r, double *s, int64_t nfree) {
     TRY(precondition(h, h->cr, h->cs));
     TRY(full_to_free(h, h->cs, s, "s"));
     TRY(sync(h));
-    return check_tc(h);
+    return check_waits(h);
 }
 
 int tosp_solve_mg(tosp_handle *h, double *x, const double *f, int64_t nfree, int32_t *it, double *relres) {
@@ -1805,7 +1807,7 @@ int tosp_time_operator(tosp_handle *h, int32_t precision, int32_t reps, double *
         return TOSP_ERR_STATE;
     }
     if (precision == 2 && !h->cg32) {
-        h->err = "the CG's tensor-core product exists only on handles created with cg_product 1";
+        h->err = "the CG's FP32 product exists only on handles created with cg_product 1";
         return TOSP_ERR_STATE;
     }
     const Grid &g0 = h->lev[0].g;
@@ -1815,24 +1817,15 @@ int tosp_time_operator(tosp_handle *h, int32_t precision, int32_t reps, double *
     double total = 0.0;
     for (int r = 0; r < reps; ++r) {
         if (precision == TOSP_PREC_FP64) {
-            CK(cudaMemsetAsync(h->cq, 0, sizeof(double) * g0.ndof, h->stream));
             CK(cudaEventRecord(a, h->stream));
-            launch_fine64(h, h->cd, h->cq);
+            TRY(fine_apply64(h, h->cd, h->cq));
         } else if (precision == 2) {
-            CK(cudaMemsetAsync(h->cq32, 0, sizeof(float) * g0.ndof, h->stream));
             CK(cudaEventRecord(a, h->stream));
-            launch_fine_apply_tc_w32(h->cd32, h->cq32, h->d_w32, h->lev[0].fm, h->d_tcimg32, h->fg, h->n, h->d_tcerr,
-                                     h->stream);
+            TRY(fine_apply_cg32(h, h->cd32, h->cq32));
         } else {
             Level &F = h->lev[0];
-            CK(cudaMemsetAsync(F.t, 0, sizeof(float) * g0.ndof, h->stream));
             CK(cudaEventRecord(a, h->stream));
-            if (h->d_tcimg)
-                launch_fine_apply_tc((const float *)F.x, (float *)F.t, h->d_wbf, F.fm, h->d_tcimg, h->fg, h->n,
-                                     h->d_tcerr, h->stream);
-            else
-                launch_fine_apply<float, __nv_bfloat16>((const float *)F.x, (float *)F.t, h->d_wbf, F.fm, h->d_kt32,
-                                                        h->fg, h->n, h->stream);
+            TRY(fine_apply<float>(h, (const float *)F.x, (float *)F.t));
         }
         CKL();
         CK(cudaEventRecord(b, h->stream));
@@ -1844,7 +1837,7 @@ int tosp_time_operator(tosp_handle *h, int32_t precision, int32_t reps, double *
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     *ms_per_launch = total / reps;
-    return check_tc(h);
+    return check_waits(h);
 }
 
 int tosp_inject_wait_fault(tosp_handle *h, int32_t polls, int32_t skip_block) {

@@ -36,47 +36,14 @@ inline Grid make_grid(int nelx, int nely, int nelz) {
     return g;
 }
 
-// Element-brick tiling of the fine-level operator: a CTA owns BX x BY x BZ
-// elements (y fastest) and the (BX+1)(BY+1)(BZ+1) nodes around them.
-constexpr int BX = 4, BY = 8, BZ = 4;
-constexpr int BRICK_ELEMS = BX * BY * BZ;            // 128 threads, one element each
-constexpr int NBX = BX + 1, NBY = BY + 1, NBZ = BZ + 1;
-constexpr int BRICK_NODES = NBX * NBY * NBZ;         // 225
 constexpr int KE_PACK = 300;                          // upper triangle of a 24x24 block
 
-// Order of the 300 upper-triangle entries (i <= j) in the fine operator's
-// block layout: diagonal by diagonal (d = j - i = 0..23), and within a
-// diagonal even i first, then odd i, so that consecutive entries never update
-// the same output (the updates y_i += k u_j, y_j += k u_i are dependent
-// through y otherwise).
-__host__ __device__ constexpr int pair_d(int t) {
-    int d = 0;
-    while (t >= 24 - d) {
-        t -= 24 - d;
-        ++d;
-    }
-    return d;
-}
-__host__ __device__ constexpr int pair_i(int t) {
-    const int d = pair_d(t);
-    int r = t;
-    for (int e = 0; e < d; ++e) r -= 24 - e;
-    const int neven = (24 - d + 1) / 2;
-    return r < neven ? 2 * r : 2 * (r - neven) + 1;
-}
-__host__ __device__ constexpr int pair_j(int t) { return pair_i(t) + pair_d(t); }
-__host__ __device__ constexpr int pair_index_diag(int i) { return (i % 2 == 0) ? i / 2 : 12 + i / 2; }
 // Row-major packed index of (i, j), i <= j (Galerkin build, Grad).
 __host__ __device__ constexpr int pair_rowmajor(int i, int j) { return i * 24 - i * (i - 1) / 2 + (j - i); }
 
 struct FineGeom {
     Grid g;
     int nelx_d, nely_d;        // density mesh (n x finer)
-    int nbx, nby, nbz;         // bricks per direction
-    int64_t nbricks;
-    // per brick: 1 when one of its nodes has a fixed dof (the write-out then
-    // reads the free-dof mask); null: every brick reads it
-    const uint8_t *bfix;
 };
 
 // Coarse-level stencil: 27 neighbour blocks of 3x3 per node, stored
@@ -104,37 +71,50 @@ void filter_taps(double rmin, double el, double eh, double ew, int opfilter, std
 void launch_simp(const double *rho, double *w64, __nv_bfloat16 *wbf, double *wq, float *w32, int64_t n, double p,
                  double emin, double E, cudaStream_t st);
 
-// Fine MR operator y = K(w) x (y must be zeroed by the caller; fixed dofs of
-// y stay zero).  kt: the n^3 blocks pair-major, see fine_nsp.
-template <typename T, typename TW>
-void launch_fine_apply(const T *x, T *y, const TW *w, const uint8_t *freemask, const T *kt, const FineGeom &fg,
-                       int n, cudaStream_t st);
+// Constants of the modal element product (fine_modal.cuh): trace factors
+// t[c] = el / h_c, and the factors with which the Gram products of the trace
+// (kt), the normal strains (kn) and the shear strains (s1 on component c, s2
+// on component d of the pair; sr = h_d / h_c) enter the gradient.
+template <typename T>
+struct ModalCoef {
+    T t[3], kt[3], kn[3], sr[3], s1[3], s2[3];
+};
+ModalCoef<double> modal_coef(double el, double eh, double ew, double nu, int n);
+
+// What a product of the finest operator does with K x at the owned nodes.
+enum FineMode : int {
+    FINE_APPLY = 0,   // out = K x
+    FINE_RESID = 1,   // out = b - K x
+    FINE_JACOBI = 2,  // out = x + invd (b - K x)
+    FINE_OUT = 3,     // FP64 out = x + invd (r - K x) (r FP64), r'out -> o0, r'so -> o1
+    FINE_DOT = 4,     // out = K x, r'(K x) -> o0 (r FP64: x before its rounding)
+};
+// Tile of the marching product: EX x EY element columns per block (EY along
+// y), LZ node planes per block, and the grid.
+struct FinePlan {
+    int ey = 0, ex = 0, lz = 0, ty = 0, tx = 0, tz = 0;
+    int blocks() const { return ty * tx * tz; }
+};
+FinePlan fine_plan(const Grid &g, int n, int elem_bytes);
+template <typename T>
+struct FineArgs {
+    const T *x = nullptr;
+    void *out = nullptr;
+    const uint8_t *fm = nullptr;      // free-dof mask
+    const uint8_t *fixed = nullptr;   // per block of the plan: owns a fixed dof (null: every block reads fm)
+    const T *b = nullptr, *invd = nullptr;
+    const double *r = nullptr, *so = nullptr;
+    double *part = nullptr, *o0 = nullptr, *o1 = nullptr;   // part: 2 * blocks + 1
+};
+// Marks the blocks of a plan that own a fixed dof (FineArgs::fixed).
+void launch_fine_fixed(const uint8_t *fm, const Grid &g, const FinePlan &plan, uint8_t *flag, cudaStream_t st);
+template <typename T, typename WT>
+void launch_fine_modal(int n, FineMode mode, const FineArgs<T> &a, const WT *w, const FineGeom &fg,
+                       const FinePlan &plan, const ModalCoef<T> &k, cudaStream_t st);
+
 // y += diag(K(w)) (y zeroed by the caller); ke64: row-major packed blocks.
 void launch_fine_diag(double *y, const double *w, const uint8_t *freemask, const double *ke64, const FineGeom &fg,
                       int n, cudaStream_t st);
-// Stride of the pair-major block layout: entry t of block s at kt[t*nsp + s].
-int fine_nsp(int n, int elem_bytes);
-// The operator's block table from the row-major packed blocks (n = 2: the
-// Walsh-Hadamard modes; otherwise pair-major with stride fine_nsp).
-void fine_block_table(const std::vector<double> &packed_rowmajor, int n, int elem_bytes, std::vector<double> &kt);
-void fine_mr2_const_table(const std::vector<double> &kt_padded, int elem_bytes, std::vector<double> &out);
-void launch_fine_apply64_const(const double *x, double *y, const double *w, const uint8_t *freemask,
-                               const double *ktab, const FineGeom &fg, cudaStream_t st);
-// Tensor-core finest operator of the mixed V-cycle (MR factor n = 1, 2, 3):
-// whether the kernel serves the mesh (its factor staging needs n * nely even),
-// the B operand image (FP16 pieces of the scaled blocks, canonical
-// shared-memory layout, then the block scale) and the launch.
-bool fine_tc_supported(int n, int nely);
-void fine_tc_image(const std::vector<double> &packed_rowmajor, int n, std::vector<uint16_t> &img);
-void launch_fine_apply_tc(const float *x, float *y, const __nv_bfloat16 *w, const uint8_t *fm, const void *bimg,
-                          const FineGeom &fg, int n, int *err, cudaStream_t st);
-// The same product with FP32 SIMP factors and the blocks in three FP16 pieces
-// (the CG's product of cg_product 1), with its own B image.
-bool fine_tc_w32_supported(int n);
-void fine_tc_image_w32(const std::vector<double> &packed_rowmajor, int n, std::vector<uint16_t> &img);
-void launch_fine_apply_tc_w32(const float *x, float *y, const float *w, const uint8_t *fm, const void *bimg,
-                              const FineGeom &fg, int n, int *err, cudaStream_t st);
-
 // Sensitivities g0 (I/Grad.m:24-49), zero for elements not in freeDensG.
 void launch_grad(const double *u, const double *rho, const uint8_t *free_elem, const double *kepack,
                  double *g0, const FineGeom &fg, int n, double p, double emin, double E, cudaStream_t st);
@@ -157,16 +137,9 @@ void launch_assemble_stencil(const double *Ae, const uint8_t *freemask, const Gr
 template <typename T>
 void launch_stencil(const T *st_vals, const T *x, const T *b, const T *invdiag, T *y, const Grid &g,
                     int mode, bool node_major, cudaStream_t st);
-// Fine-level helpers: y = b - t ; x = x + invD (b - t) ; x = invD b
+// First sweep from zero: x = invD b.
 template <typename T>
-void launch_residual(const T *b, const T *t, T *r, int64_t n, cudaStream_t st);
-template <typename T>
-void launch_jacobi_update(T *x, const T *b, const T *t, const T *invdiag, int64_t n, int first,
-                          cudaStream_t st);
-// Last sweep of a cycle written in FP64: out = x + invD (b - t) (computed in T).
-template <typename T>
-void launch_jacobi_out(double *out, const T *x, const T *b, const T *t, const T *invdiag, int64_t n,
-                       cudaStream_t st);
+void launch_jacobi_zero(T *x, const T *b, const T *invdiag, int64_t n, cudaStream_t st);
 template <typename T>
 void launch_invert_diag(const T *diag, const uint8_t *freemask, T *invdiag, double omega, int64_t n,
                         cudaStream_t st);
@@ -179,10 +152,6 @@ void launch_prolong(const T *xc, T *xf, const uint8_t *freemask_f, const Grid &g
 template <typename T>
 void launch_restrict(const T *rf, T *bc, const uint8_t *freemask_c, const Grid &gf, const Grid &gc,
                      cudaStream_t st, const T *invd_c = nullptr, T *xc = nullptr);
-// Restriction of the residual bf - tf (the level-0 residual fused in).
-template <typename T>
-void launch_restrict_res(const T *bf, const T *tf, T *bc, const uint8_t *freemask_c, const Grid &gf,
-                         const Grid &gc, cudaStream_t st, const T *invd_c = nullptr, T *xc = nullptr);
 void launch_coarse_freemask(const uint8_t *freemask_f, uint8_t *freemask_c, const Grid &gf,
                             const Grid &gc, cudaStream_t st);
 
@@ -270,7 +239,6 @@ void launch_convert(const TI *a, TO *b, int64_t n, cudaStream_t st);
 // Deterministic dot products: out[0] = sum a*b (fixed reduction tree).
 constexpr int RED_BLOCKS = 592;
 void launch_dot(const double *a, const double *b, int64_t n, double *partials, double *out, cudaStream_t st);
-void launch_dot(const double *a, const float *b, int64_t n, double *partials, double *out, cudaStream_t st);
 // a'b -> out0 and a'c -> out1 in one pass (partials: 2 * RED_BLOCKS).
 void launch_dot2(const double *a, const double *b, const double *c, int64_t n, double *partials, double *out0,
                  double *out1, cudaStream_t st);
@@ -278,11 +246,6 @@ void launch_dot2(const double *a, const double *b, const double *c, int64_t n, d
 void launch_pcg_direction(double *d, const double *s, double *sold, const double *scal, int64_t n, int mode,
                           double *x, cudaStream_t st, float *d32 = nullptr);
 void launch_pcg_finish(double *x, const double *d, const double *scal, int64_t n, cudaStream_t st);
-// launch_jacobi_out with the CG's dots r's (-> out0) and r's_old (-> out1,
-// when so is given) of the new s in the same pass.
-template <typename T>
-void launch_jacobi_out_dot(double *out, const T *x, const T *b, const T *t, const T *invd, int64_t n, const double *r,
-                           const double *so, double *partials, double *out0, double *out1, cudaStream_t st);
 void launch_pcg_update(double *r, const double *q, double *scal, double *partials, int64_t n, cudaStream_t st,
                        float *b0 = nullptr, const float *invd0 = nullptr, float *x0 = nullptr);
 void launch_pcg_update(double *r, const float *q, double *scal, double *partials, int64_t n, cudaStream_t st,

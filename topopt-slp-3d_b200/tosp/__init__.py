@@ -265,15 +265,15 @@ class Solver:
 
     def KelemProdMixed(self, x):
         """K(rho) x by the mixed V-cycle's finest operator (FP32 vectors, BF16
-        SIMP factors; tensor-core sub-cell products when n * nely is even)."""
+        SIMP factors)."""
         x = np.ascontiguousarray(x, dtype=np.float64)
         y = np.empty_like(x)
         self._check(_lib.tosp_kelem_prod_mixed(self.h, _ptr(x), _ptr(y), x.size))
         return y
 
     def KelemProdCG32(self, x):
-        """K(rho) x by the CG's product of ``mg.cg_product = 1`` (tensor cores,
-        FP32 SIMP factors and vectors)."""
+        """K(rho) x by the CG's product of ``mg.cg_product = 1`` (FP32
+        SIMP factors and vectors)."""
         x = np.ascontiguousarray(x, dtype=np.float64)
         y = np.empty_like(x)
         self._check(_lib.tosp_kelem_prod_cg32(self.h, _ptr(x), _ptr(y), x.size))

@@ -4,19 +4,14 @@
 // amd + sparse chol and applies eH = R\(R'\rH(perm)) in every cycle
 // (I/SetupGMG.m:51-59, I/VCycle.m:40).  Here the coarsest matrix is assembled
 // densely (fixed dofs decoupled with a unit diagonal, padded to a multiple of
-// 32 with identity) and inverted once per setup in place by a blocked
+// DB with identity) and inverted once per setup in place by a blocked
 // symmetric sweep, so that each cycle's coarse solve is a single FP64 GEMV
 // that runs from L2.
 #include "tosp_internal.h"
 
 namespace tosp {
 
-constexpr int TS = 32;
-
-__global__ void k_dense_zero(double *A, int64_t nn) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nn; i += (int64_t)gridDim.x * blockDim.x)
-        A[i] = 0.0;
-}
+constexpr int DB = DENSE_BLOCK;
 
 __global__ void k_dense_scatter(const double *__restrict__ Ae, const uint8_t *__restrict__ fm, Grid g, double *A,
                                 int64_t npad) {
@@ -40,138 +35,343 @@ __global__ void k_dense_unitdiag(double *A, const uint8_t *fm, int64_t n, int64_
 
 void launch_dense_assemble(const double *Ae, const uint8_t *freemask, const Grid &g, double *A, int64_t npad,
                            cudaStream_t st) {
-    k_dense_zero<<<1024, 256, 0, st>>>(A, npad * npad); count_launch();
+    cudaMemsetAsync(A, 0, sizeof(double) * npad * npad, st);
     k_dense_scatter<<<1024, 256, 0, st>>>(Ae, freemask, g, A, npad); count_launch();
     k_dense_unitdiag<<<64, 256, 0, st>>>(A, freemask, g.ndof, npad); count_launch();
 }
 
 // --- blocked symmetric sweep (block Gauss-Jordan) ----------------------------
-// Sweeping block k of a symmetric matrix:  P = A_kk,  C_i = A_ik P^{-1},
-//   A_ij -= C_i A_kj (i, j != k),  A_ik = C_i,  A_kj = C_j',  A_kk = -P^{-1}.
+// Sweeping block k of a symmetric matrix:  P = A_kk,  G_i = A_ik,
+// C_i = G_i P^{-1},
+//   A_ij -= C_i G_j' (i, j != k),  A_ik = C_i,  A_kk = -P^{-1}.
 // After all blocks the array holds -A^{-1}.  Every pivot block is a Schur
 // complement of the SPD matrix (a leading-block Cholesky factor exists), so no
-// pivoting is needed.  Each step is one small pivot inversion plus an
-// embarrassingly parallel rank-32 update of the whole matrix.
+// pivoting is needed.  Only the tiles on and below the diagonal are kept up to
+// date; the last pass mirrors and negates them.
+//
+// Two launches per block of 64: the panel (G and C, stored transposed so that
+// the update reads rows), and the rank-64 update by 64 x 64 tiles, whose first
+// block takes the next pivot's tile and inverts it while the others work.
+// With blocks of 32, four launches each and the pivot on its own, the chain of
+// small launches was the time: 1 911 dofs 3.0 -> 1.0 ms, 4 158 dofs
+// 17 -> 4.0 ms (FP64 floor of the half updates, n^3 / 2 FMAs: 0.19 and 1.9 ms).
+//
+// The products run as FP64 matrix instructions (8 x 8 x 4): with FMAs and 4 x 4
+// values per thread the shared-memory reads, four wavefronts for a 16-byte load
+// whatever it broadcasts, held the update at 44 % of the FP64 rate.
 
-// P^{-1} of the 32x32 pivot block by a scalar sweep in shared memory.
-__global__ void k_sweep_pivot(const double *A, int64_t npad, int k, double *Pinv, int *info) {
-    __shared__ double S[TS][TS + 1];
-    __shared__ double rd;
-    const int r = threadIdx.y, c = threadIdx.x;   // 32 x 32
-    S[r][c] = A[(int64_t)(k * TS + r) * npad + k * TS + c];
-    for (int p = 0; p < TS; ++p) {
-        __syncthreads();
-        if (r == 0 && c == 0) {   // one division per step, shared by all threads
-            const double d = S[p][p];
-            if (!(d > 0.0)) atomicExch(info, 1 + k * TS + p);
-            rd = 1.0 / d;
+// D += A B, A 8 x 4 (lane: row l / 4, column l % 4), B 4 x 8 (row l % 4, column
+// l / 4), D 8 x 8 (row l / 4, columns 2 (l % 4) and the next).
+__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(d[0]), "+d"(d[1])
+        : "d"(a), "d"(b));
+}
+
+// A 64 x 64 tile of eight warps: warp w holds rows 16 (w / 2) .. + 15 and columns
+// 32 (w % 2) .. + 31 as 2 x 4 blocks of 8 x 8; value (f, g, h) of thread t:
+__device__ __forceinline__ int tile_row(int t, int f) { return (t >> 6) * 16 + f * 8 + ((t & 31) >> 2); }
+__device__ __forceinline__ int tile_col(int t, int g) { return ((t >> 5) & 1) * 32 + g * 8 + 2 * (t & 3); }   // and + 1
+
+// Row stride of shared k-major operands: 2 TS % 32 == 8 spreads a fragment's
+// 4 x 4 half over all banks.
+constexpr int TS = DB + 4;
+
+// acc += X' Y over the first `rows` rows (a multiple of 4) of two k-major tiles.
+__device__ __forceinline__ void tile_mma(const double *X, const double *Y, int rows, int t, double (&acc)[2][4][2]) {
+    const int l = t & 31;
+    const double *xr = X + (l & 3) * TS + (t >> 6) * 16 + (l >> 2);
+    const double *yr = Y + (l & 3) * TS + ((t >> 5) & 1) * 32 + (l >> 2);
+#pragma unroll 4
+    for (int q = 0; q < rows; q += 4) {
+        double a[2], b[4];
+#pragma unroll
+        for (int f = 0; f < 2; ++f) a[f] = xr[q * TS + 8 * f];
+#pragma unroll
+        for (int g = 0; g < 4; ++g) b[g] = yr[q * TS + 8 * g];
+#pragma unroll
+        for (int f = 0; f < 2; ++f)
+#pragma unroll
+            for (int g = 0; g < 4; ++g) mma_f64(acc[f][g], a[f], b[g]);
+    }
+}
+
+__device__ __forceinline__ void dense_cp16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+// P^{-1} of a tile V held by the block, swept by sub-blocks of 8: their eight
+// rows R go through shared memory (by symmetry they serve as the columns), one
+// warp inverts the 8 x 8 pivot in registers, and all warps apply
+// V += R' (-Q R) with the inverse Q.  (A scalar sweep, with a barrier and a
+// division by all threads per pivot, took 40 us; this takes 16.)
+constexpr int SB = 8;
+struct TileInverse {
+    double R[2][SB * TS], QR[SB * TS], Q[SB][SB];   // QR: -Q R
+};
+
+// 1 / d from the hardware's approximation q (about 20 bits): with e = 1 - d q,
+// 1 / d = q / (1 - e) = q (1 + e + e^2 + ...), cut after e^2: a shorter
+// chain than a division, to within the last bits.
+__device__ __forceinline__ double series_rcp(double d) {
+    double q;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(q) : "d"(d));
+    const double e = fma(-d, q, 1.0);
+    return fma(q, fma(e, e, e), q);
+}
+
+// Inverse of the symmetric 8 x 8 block at R[.][p0 + .] by one warp: lane l holds
+// (l / 4, 2 (l % 4)) and the element to its right.
+__device__ __forceinline__ void block_inverse(const double *R, double (&Q)[SB][SB], int p0, int dof0, int *info) {
+    const int l = threadIdx.x, r = l >> 2, c = 2 * (l & 3);
+    double v0 = R[r * TS + p0 + c], v1 = R[r * TS + p0 + c + 1];
+#pragma unroll
+    for (int p = 0; p < SB; ++p) {
+        const double d = __shfl_sync(0xffffffffu, (p & 1) ? v1 : v0, 4 * p + p / 2);
+        const double fr = __shfl_sync(0xffffffffu, (p & 1) ? v1 : v0, (l & ~3) + p / 2);   // (r, p)
+        const double c0 = __shfl_sync(0xffffffffu, v0, 4 * p + (l & 3));                   // (p, c)
+        const double c1 = __shfl_sync(0xffffffffu, v1, 4 * p + (l & 3));
+        if (l == 0 && !(d > 0.0)) atomicCAS(info, 0, 1 + dof0 + p0 + p);
+        // (products before the reciprocal: the chain from pivot to pivot is the time)
+        const double q = series_rcp(d), f0 = fr * c0, f1 = fr * c1;
+        v0 = r == p ? (c == p ? -q : c0 * q) : (c == p ? fr * q : fma(-f0, q, v0));
+        v1 = r == p ? (c + 1 == p ? -q : c1 * q) : (c + 1 == p ? fr * q : fma(-f1, q, v1));
+    }
+    Q[r][c] = -v0;
+    Q[r][c + 1] = -v1;
+}
+
+__device__ __forceinline__ void tile_inverse(double (&v)[2][4][2], TileInverse &w, int t, int dof0, double *Pinv,
+                                             int *info) {
+    const int l = t & 31;
+#pragma unroll 1
+    for (int s = 0; s < DB / SB; ++s) {
+        const int p0 = s * SB;
+        double *R = w.R[s & 1];
+        // which of this warp's 8-row and 8-column groups are the block's (as bits:
+        // an index into v would put it into local memory)
+        const unsigned rows = (t >> 6) == (s >> 1) ? 1u << (s & 1) : 0u;
+        const unsigned cols = ((t >> 5) & 1) == (s >> 2) ? 1u << (s & 3) : 0u;
+#pragma unroll
+        for (int f = 0; f < 2; ++f) {
+            if (!((rows >> f) & 1u)) continue;
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+                *reinterpret_cast<double2 *>(R + (l >> 2) * TS + tile_col(t, g)) = make_double2(v[f][g][0], v[f][g][1]);
         }
         __syncthreads();
-        const double q = rd;
-        double v;
-        if (r == p && c == p) v = -q;
-        else if (c == p) v = S[r][p] * q;
-        else if (r == p) v = S[p][c] * q;
-        else v = S[r][c] - S[r][p] * (S[p][c] * q);
+        if (t < 32) block_inverse(R, w.Q, p0, dof0, info);
         __syncthreads();
-        S[r][c] = v;
-    }
-    __syncthreads();
-    Pinv[r * TS + c] = -S[r][c];
-}
-
-// C_i = A_ik P^{-1} for every row block i != k.
-__global__ void k_sweep_panel(const double *A, int64_t npad, int k, const double *Pinv, double *C) {
-    __shared__ double At[TS][TS + 1];
-    __shared__ double Pt[TS][TS + 1];
-    const int i = blockIdx.x;
-    if (i == k) return;
-    const int r = threadIdx.y, c = threadIdx.x;
-    At[r][c] = A[(int64_t)(i * TS + r) * npad + k * TS + c];
-    Pt[r][c] = Pinv[r * TS + c];
-    __syncthreads();
-    double v = 0.0;
-#pragma unroll 8
-    for (int q = 0; q < TS; ++q) v += At[r][q] * Pt[q][c];
-    C[(int64_t)(i * TS + r) * TS + c] = v;
-}
-
-// A_ij -= C_i A_kj for all entries outside row and column block k: a
-// rank-32 update by 64 x 64 tiles, 256 threads, 4 x 4 outputs per thread
-// (rows ty + 16 a, columns tx + 16 b) from shared copies of the tile's C rows
-// and A_k columns.
-constexpr int UT = 64;
-__global__ void __launch_bounds__(256) k_sweep_update(double *A, int64_t npad, int k, const double *C, int ntile) {
-    __shared__ double Cs[UT][TS + 1];
-    __shared__ double Rs[TS][UT + 1];
-    const int ti = blockIdx.x / ntile, tj = blockIdx.x % ntile;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int row0 = ti * UT, col0 = tj * UT;
-    for (int e = threadIdx.x; e < UT * TS; e += 256) {
-        const int rr = e / TS, q = e % TS;
-        const int64_t gr = row0 + rr;
-        Cs[rr][q] = gr < npad ? C[gr * TS + q] : 0.0;
-        const int q2 = e / UT, cc = e % UT;
-        const int64_t gc = col0 + cc;
-        Rs[q2][cc] = gc < npad ? A[(int64_t)(k * TS + q2) * npad + gc] : 0.0;
-    }
-    __syncthreads();
-    double acc[4][4] = {};
-#pragma unroll 8
-    for (int q = 0; q < TS; ++q) {
-        double cv[4], rv[4];
+        {
+            // -Q R: warp w makes columns 8 w .. + 7
+            const int c0 = (t >> 5) * 8;
+            double o[2] = {0.0, 0.0};
 #pragma unroll
-        for (int a = 0; a < 4; ++a) cv[a] = Cs[ty + 16 * a][q];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) rv[b] = Rs[q][tx + 16 * b];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) acc[a][b] = fma(cv[a], rv[b], acc[a][b]);
-    }
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const int64_t gr = row0 + ty + 16 * a;
-        if (gr >= npad || gr / TS == k) continue;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int64_t gc = col0 + tx + 16 * b;
-            if (gc >= npad || gc / TS == k) continue;
-            A[gr * npad + gc] -= acc[a][b];
+            for (int k = 0; k < SB; k += 4)
+                mma_f64(o, -w.Q[l >> 2][k + (l & 3)], R[(k + (l & 3)) * TS + c0 + (l >> 2)]);
+            *reinterpret_cast<double2 *>(w.QR + (l >> 2) * TS + c0 + 2 * (l & 3)) = make_double2(o[0], o[1]);
         }
+        __syncthreads();
+        tile_mma(R, w.QR, SB, t, v);
+        // the block's rows Q R, its columns (Q R)', the block itself -Q
+#pragma unroll
+        for (int f = 0; f < 2; ++f)
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int r = l >> 2, c = 2 * (l & 3) + h;
+                    const bool pr = (rows >> f) & 1u, pc = (cols >> g) & 1u;
+                    if (pr) v[f][g][h] = pc ? -w.Q[r][c] : -w.QR[r * TS + tile_col(t, g) + h];
+                    else if (pc) v[f][g][h] = -w.QR[c * TS + tile_row(t, f)];
+                }
     }
+#pragma unroll
+    for (int f = 0; f < 2; ++f)
+#pragma unroll
+        for (int g = 0; g < 4; ++g)
+            *reinterpret_cast<double2 *>(Pinv + tile_row(t, f) * DB + tile_col(t, g)) =
+                make_double2(-v[f][g][0], -v[f][g][1]);
 }
 
-// Column and row blocks of k: A_ik = C_i, A_ki = C_i', A_kk = -P^{-1}.
-__global__ void k_sweep_setrc(double *A, int64_t npad, int k, const double *C, const double *Pinv) {
-    const int i = blockIdx.x;
-    const int r = threadIdx.y, c = threadIdx.x;
+__global__ void __launch_bounds__(256) k_sweep_first(const double *A, int64_t npad, double *Pinv, int *info) {
+    __shared__ __align__(16) TileInverse w;
+    const int t = threadIdx.x;
+    double v[2][4][2];
+#pragma unroll
+    for (int f = 0; f < 2; ++f)
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            const double2 o = *reinterpret_cast<const double2 *>(A + tile_row(t, f) * npad + tile_col(t, g));
+            v[f][g][0] = o.x;
+            v[f][g][1] = o.y;
+        }
+    tile_inverse(v, w, t, 0, Pinv, info);
+}
+
+// PR rows of row tile i of block column k: Gt[q][i] = G_i', Ct[c][i] = C_i'
+// (64 x npad each), and the column's new values.  Warp w makes columns 8 w .. + 7.
+constexpr int PR = 16, GS = PR + 4;
+constexpr int PANEL_SMEM = (DB * TS + DB * GS) * (int)sizeof(double);
+__global__ void __launch_bounds__(256) k_sweep_panel(double *A, int64_t npad, int k, const double *__restrict__ Pinv,
+                                                     double *__restrict__ Gt, double *__restrict__ Ct) {
+    extern __shared__ __align__(16) double sm[];
+    double *P = sm, *G = sm + DB * TS;                    // P[q][c], G[q][r]
+    const int t = threadIdx.x, i = blockIdx.x / (DB / PR), r0 = i * DB + (int)(blockIdx.x % (DB / PR)) * PR;
     if (i == k) {
-        A[(int64_t)(k * TS + r) * npad + k * TS + c] = -Pinv[r * TS + c];
+        for (int e = t; e < PR * DB; e += 256)
+            A[(int64_t)(r0 + e / DB) * npad + k * DB + e % DB] = -Pinv[(r0 - k * DB) * DB + e];
+        return;
+    }
+#pragma unroll
+    for (int u = 0; u < DB * DB / 2 / 256; ++u) {
+        const int e = t + 256 * u, q = e / (DB / 2), c = 2 * (e % (DB / 2));
+        dense_cp16(P + q * TS + c, Pinv + q * DB + c);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    double gv[PR * DB / 256];
+#pragma unroll
+    for (int u = 0; u < PR * DB / 256; ++u) {
+        const int e = t + 256 * u;
+        gv[u] = i > k ? A[(int64_t)(r0 + e / DB) * npad + k * DB + e % DB]     // stored as (i, k)
+                      : A[(int64_t)(k * DB + e / PR) * npad + r0 + e % PR];    // stored as (k, i)
+    }
+#pragma unroll
+    for (int u = 0; u < PR * DB / 256; ++u) {
+        const int e = t + 256 * u;
+        if (i > k) G[(e % DB) * GS + e / DB] = gv[u];
+        else G[(e / PR) * GS + e % PR] = gv[u];
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < PR * DB / 256; ++u) {
+        const int e = t + 256 * u, q = e / PR, rr = e % PR;
+        Gt[(int64_t)q * npad + r0 + rr] = G[q * GS + rr];
+    }
+    // C[r][c] = sum_q G[q][r] P[q][c]
+    const int l = t & 31, c0 = (t >> 5) * 8;
+    double acc[2][2] = {};
+#pragma unroll
+    for (int q = 0; q < DB; q += 4) {
+        const double b = P[(q + (l & 3)) * TS + c0 + (l >> 2)];
+#pragma unroll
+        for (int f = 0; f < 2; ++f) mma_f64(acc[f], G[(q + (l & 3)) * GS + 8 * f + (l >> 2)], b);
+    }
+    __syncthreads();
+    double *T = sm;                                       // C[r][c], over P
+#pragma unroll
+    for (int f = 0; f < 2; ++f)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) T[(8 * f + (l >> 2)) * (DB + 1) + c0 + 2 * (l & 3) + h] = acc[f][h];
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < PR * DB / 256; ++u) {
+        const int e = t + 256 * u, c = e / PR, rr = e % PR;
+        Ct[(int64_t)c * npad + r0 + rr] = T[rr * (DB + 1) + c];
+        if (i < k) A[(int64_t)(k * DB + c) * npad + r0 + rr] = T[rr * (DB + 1) + c];
+        else A[(int64_t)(r0 + e / DB) * npad + k * DB + e % DB] = T[e / DB * (DB + 1) + e % DB];
+    }
+}
+
+// A_ij -= C_i G_j' for the tiles i >= j outside row and column k.  Block 0 takes
+// tile (k + 1, k + 1) and inverts it.
+constexpr int DQ = 16;   // rows of Ct and Gt staged at a time (two stages)
+__global__ void __launch_bounds__(256, 4) k_sweep_update(double *A, int64_t npad, int nt, int k,
+                                                         const double *__restrict__ Gt, const double *__restrict__ Ct,
+                                                         double *Pinv, int *info) {
+    __shared__ __align__(16) union {
+        double st[2][2][DQ * TS];
+        TileInverse w;
+    } sm;
+    const int t = threadIdx.x;
+    int i, j;
+    if (blockIdx.x == 0) {
+        i = j = k + 1;
+        if (i >= nt) return;
     } else {
-        const double v = C[(int64_t)(i * TS + r) * TS + c];
-        A[(int64_t)(i * TS + r) * npad + k * TS + c] = v;
-        A[(int64_t)(k * TS + c) * npad + i * TS + r] = v;
+        const int e = (int)blockIdx.x - 1;
+        i = (int)((sqrt(8.0 * e + 1.0) - 1.0) * 0.5);
+        while ((i + 1) * (i + 2) / 2 <= e) ++i;
+        while (i * (i + 1) / 2 > e) --i;
+        j = e - i * (i + 1) / 2;
+        if (i == k || j == k || (i == j && i == k + 1)) return;
+    }
+    auto stage = [&](int c) {
+        double *X = sm.st[c & 1][0], *Y = sm.st[c & 1][1];
+#pragma unroll
+        for (int u = 0; u < DQ * DB / 2 / 256; ++u) {
+            const int e = t + 256 * u, q = e / (DB / 2), col = 2 * (e % (DB / 2));
+            dense_cp16(X + q * TS + col, Ct + (int64_t)(c * DQ + q) * npad + i * DB + col);
+            dense_cp16(Y + q * TS + col, Gt + (int64_t)(c * DQ + q) * npad + j * DB + col);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    double acc[2][4][2] = {};
+    stage(0);
+#pragma unroll
+    for (int c = 0; c < DB / DQ; ++c) {
+        if (c + 1 < DB / DQ) {
+            stage(c + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        tile_mma(sm.st[c & 1][0], sm.st[c & 1][1], DQ, t, acc);
+        __syncthreads();
+    }
+#pragma unroll
+    for (int f = 0; f < 2; ++f)
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            double2 *p = reinterpret_cast<double2 *>(A + (int64_t)(i * DB + tile_row(t, f)) * npad + j * DB +
+                                                     tile_col(t, g));
+            double2 o = *p;
+            o.x -= acc[f][g][0];
+            o.y -= acc[f][g][1];
+            *p = o;
+            acc[f][g][0] = o.x;
+            acc[f][g][1] = o.y;
+        }
+    if (blockIdx.x == 0) tile_inverse(acc, sm.w, t, i * DB, Pinv, info);
+}
+
+// A = -(lower tiles), mirrored.
+__global__ void __launch_bounds__(256) k_sweep_mirror(double *A, int64_t npad) {
+    __shared__ double T[DB][DB + 1];
+    const int e0 = (int)blockIdx.x, t = threadIdx.x;
+    int i = (int)((sqrt(8.0 * e0 + 1.0) - 1.0) * 0.5);
+    while ((i + 1) * (i + 2) / 2 <= e0) ++i;
+    while (i * (i + 1) / 2 > e0) --i;
+    const int j = e0 - i * (i + 1) / 2;
+    for (int e = t; e < DB * DB; e += 256) {
+        double *p = A + (int64_t)(i * DB + e / DB) * npad + j * DB + e % DB;
+        const double v = -*p;
+        T[e / DB][e % DB] = v;
+        if (i != j) *p = v;
+    }
+    __syncthreads();
+    // a diagonal tile takes its lower half on both sides
+    for (int e = t; e < DB * DB; e += 256) {
+        const int r = e / DB, c = e % DB;
+        A[(int64_t)(j * DB + r) * npad + i * DB + c] = (i == j && c < r) ? T[r][c] : T[c][r];
     }
 }
 
-__global__ void k_negate(double *A, int64_t nn) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nn; i += (int64_t)gridDim.x * blockDim.x)
-        A[i] = -A[i];
-}
-
-int dense_sweep_inverse(double *A, double *C, double *Pinv, int64_t npad, int *d_info, cudaStream_t st) {
-    const int nb = (int)(npad / TS);
-    const int ntile = (int)((npad + UT - 1) / UT);
-    const dim3 blk(TS, TS);
+int dense_sweep_inverse(double *A, double *work, double *Pinv, int64_t npad, int *d_info, cudaStream_t st) {
+    const int nt = (int)(npad / DB), tiles = nt * (nt + 1) / 2;
+    double *Gt = work, *Ct = work + DB * npad;
+    cudaFuncSetAttribute(k_sweep_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, PANEL_SMEM);
     cudaMemsetAsync(d_info, 0, sizeof(int), st);
-    for (int k = 0; k < nb; ++k) {
-        k_sweep_pivot<<<1, blk, 0, st>>>(A, npad, k, Pinv, d_info); count_launch();
-        k_sweep_panel<<<nb, blk, 0, st>>>(A, npad, k, Pinv, C); count_launch();
-        k_sweep_update<<<ntile * ntile, 256, 0, st>>>(A, npad, k, C, ntile); count_launch();
-        k_sweep_setrc<<<nb, blk, 0, st>>>(A, npad, k, C, Pinv); count_launch();
+    k_sweep_first<<<1, 256, 0, st>>>(A, npad, Pinv, d_info); count_launch();
+    for (int k = 0; k < nt; ++k) {
+        k_sweep_panel<<<nt * (DB / PR), 256, PANEL_SMEM, st>>>(A, npad, k, Pinv, Gt, Ct); count_launch();
+        if (nt == 1) break;
+        k_sweep_update<<<1 + tiles, 256, 0, st>>>(A, npad, nt, k, Gt, Ct, Pinv, d_info); count_launch();
     }
-    k_negate<<<1024, 256, 0, st>>>(A, npad * npad); count_launch();
+    k_sweep_mirror<<<tiles, 256, 0, st>>>(A, npad); count_launch();
     return 0;
 }
 

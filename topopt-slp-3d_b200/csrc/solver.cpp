@@ -76,7 +76,7 @@ struct tosp_handle {
     // hierarchy
     std::vector<Level> lev;
     double *d_diag64 = nullptr;     // diag of the finest operator
-    double *d_Adense = nullptr, *d_sweepC = nullptr, *d_pinv = nullptr;   // coarsest: A, then A^{-1}
+    double *d_Adense = nullptr, *d_sweep = nullptr, *d_pinv = nullptr;   // coarsest: A, then A^{-1}
     int64_t ncoarse = 0, npad = 0;
     // coarsest grid by PCG (mg.opchol = 1 or the level rule's switch): FP64
     // node-major stencil, 1 / diag and the kernel's work buffers
@@ -780,7 +780,7 @@ int create_impl(tosp_handle *h, const tosp_problem *pb, const tosp_mg_params *mg
     h->dens = make_grid(pb->nelx * h->n, pb->nely * h->n, pb->nelz * h->n);
     h->ncoarse = h->mg_ok ? h->lev[ng - 1].g.ndof : 0;
     h->coarse_pcg = h->mg_ok && cpcg;
-    h->npad = h->coarse_pcg ? 0 : (h->ncoarse + 31) / 32 * 32;
+    h->npad = h->coarse_pcg ? 0 : (h->ncoarse + DENSE_BLOCK - 1) / DENSE_BLOCK * DENSE_BLOCK;
     if (h->npad > DENSE_MAX) {
         h->err = "coarsest system too large for the dense direct solve: " + std::to_string(h->ncoarse) +
                  " dofs; use more grids";
@@ -854,8 +854,8 @@ int create_impl(tosp_handle *h, const tosp_problem *pb, const tosp_mg_params *mg
         TRY(dalloc(h, &w.iters, 1));
     } else if (h->mg_ok) {
         TRY(dalloc(h, &h->d_Adense, h->npad * h->npad));
-        TRY(dalloc(h, &h->d_sweepC, h->npad * 32));
-        TRY(dalloc(h, &h->d_pinv, 32 * 32));
+        TRY(dalloc(h, &h->d_sweep, 2 * DENSE_BLOCK * h->npad));
+        TRY(dalloc(h, &h->d_pinv, DENSE_BLOCK * DENSE_BLOCK));
     }
     TRY(dalloc(h, &h->d_info, 1));
     // densities
@@ -985,7 +985,7 @@ int setup_levels(tosp_handle *h) {
     }
     launch_dense_assemble(C.Ae, C.fm, C.g, h->d_Adense, h->npad, h->stream);
     CKL();
-    dense_sweep_inverse(h->d_Adense, h->d_sweepC, h->d_pinv, h->npad, h->d_info, h->stream);
+    dense_sweep_inverse(h->d_Adense, h->d_sweep, h->d_pinv, h->npad, h->d_info, h->stream);
     CKL();
     int info = 0;
     CK(cudaMemcpyAsync(&info, h->d_info, sizeof(int), cudaMemcpyDeviceToHost, h->stream));

@@ -155,12 +155,14 @@ void launch_restrict(const T *rf, T *bc, const uint8_t *freemask_c, const Grid &
 void launch_coarse_freemask(const uint8_t *freemask_f, uint8_t *freemask_c, const Grid &gf,
                             const Grid &gc, cudaStream_t st);
 
-// Coarsest direct solve: dense SPD matrix (padded to a multiple of 32, fixed
-// dofs decoupled with a unit diagonal), explicit inverse in place by a blocked
-// symmetric sweep (C: npad x 32 workspace, Pinv: 32 x 32), GEMV.
+// Coarsest direct solve: dense SPD matrix (padded to a multiple of DENSE_BLOCK,
+// fixed dofs decoupled with a unit diagonal), explicit inverse in place by a
+// blocked symmetric sweep (work: 2 x DENSE_BLOCK x npad, Pinv: DENSE_BLOCK^2),
+// GEMV.
+constexpr int DENSE_BLOCK = 64;
 void launch_dense_assemble(const double *Ae, const uint8_t *freemask, const Grid &g, double *A,
                            int64_t npad, cudaStream_t st);
-int dense_sweep_inverse(double *A, double *C, double *Pinv, int64_t npad, int *d_info, cudaStream_t st);
+int dense_sweep_inverse(double *A, double *work, double *Pinv, int64_t npad, int *d_info, cudaStream_t st);
 template <typename T>
 void launch_dense_solve(const double *X, const T *b, T *x, int64_t n, int64_t npad, cudaStream_t st);
 

@@ -190,6 +190,79 @@ __device__ __forceinline__ void modal_stress(const T (&m)[3][8], const T (&W)[mo
     }
 }
 
+// F[t] += k sum_{p + q = t} E[p] E[q] over the monomials `in`: the energy's
+// derivative with respect to the moments.
+template <int N, typename T, typename In>
+__device__ __forceinline__ void modal_energy_gram(T k, const T (&E)[8], T (&F)[modal_moments<N>], In in) {
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+        if (!in(p)) continue;
+        const T kp = k * E[p];
+        F[modal_index<N>(p, p)] += kp * E[p];
+        if constexpr (N > 1) {
+#pragma unroll
+            for (int q = p + 1; q < 8; ++q)
+                if (in(q)) F[modal_index<N>(p, q)] += (T(2) * kp) * E[q];
+        }
+    }
+}
+
+// Energies u' KE_s u of the cells from the modes m: the products of the strain
+// coefficients gathered by moment, then the transpose of modal_weights.
+template <int N, typename T>
+__device__ __forceinline__ void modal_energies(const T (&m)[3][8], const ModalCoef<T> &k, T (&q)[N * N * N]) {
+    T E[8], F[modal_moments<N>];
+#pragma unroll
+    for (int t = 0; t < modal_moments<N>; ++t) F[t] = T(0);
+    modal_trace(m, k, E);
+    modal_energy_gram<N>(k.kt[0], E, F, [](int p) { return modal_in_trace(p); });
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+#pragma unroll
+        for (int p = 0; p < 8; ++p)
+            if (!((p >> c) & 1)) E[p] = m[c][p | (1 << c)];
+        modal_energy_gram<N>(k.kn[c], E, F, [c](int p) { return modal_in_normal(p, c); });
+    }
+#pragma unroll
+    for (int kk = 0; kk < 3; ++kk) {
+        const int c = modal_sc(kk), d = modal_sd(kk);
+        modal_shear(m, k, kk, E);
+        modal_energy_gram<N>(k.s1[kk], E, F, [c, d](int p) { return modal_in_shear(p, c, d); });
+    }
+    if constexpr (N == 1) {
+        q[0] = F[0];
+    } else if constexpr (N == 2) {
+#pragma unroll
+        for (int b = 1; b < 8; ++b)
+            F[b] *= modal_deg(b) == 1 ? T(1.5 * MODAL_R3) : (modal_deg(b) == 2 ? T(0.75) : T(1.125 * MODAL_R3));
+#pragma unroll
+        for (int bit = 1; bit < 8; bit <<= 1)
+#pragma unroll
+            for (int b = 0; b < 8; ++b)
+                if (!(b & bit)) {
+                    const T e = F[b], o = F[b | bit];
+                    F[b] = e - o;
+                    F[b | bit] = e + o;
+                }
+#pragma unroll
+        for (int s = 0; s < 8; ++s) q[s] = F[((s & 1) << 1) | ((s >> 1) & 1) | (s & 4)];
+    } else {
+#pragma unroll
+        for (int s = 1; s < 27; s *= 3)
+#pragma unroll
+            for (int b = 0; b < 27; ++b)
+                if (b / s % 3 == 0) {
+                    const T f0 = F[b], f1 = T(2.0 * MODAL_R3) * F[b + s], f2 = F[b + 2 * s];
+                    const T e = f0 + T(13.0 / 9.0) * f2;
+                    F[b] = e - f1;
+                    F[b + s] = f0 + T(1.0 / 9.0) * f2;
+                    F[b + 2 * s] = e + f1;
+                }
+#pragma unroll
+        for (int s = 0; s < 27; ++s) q[s] = F[(s / 3 % 3) + 3 * (s % 3) + 9 * (s / 9)];
+    }
+}
+
 // Two-dimensional modes (x, y) of one component on a node plane from the four
 // corner values.  FP32 keeps the low corner apart and transforms the
 // differences to it, which are exact or nearly so for the smooth fields of a

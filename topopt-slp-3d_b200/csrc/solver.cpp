@@ -71,6 +71,8 @@ struct tosp_handle {
     FilterTap *d_taps = nullptr;
     int filt_r = 0;                 // largest |offset| of the taps
     int ntaps = 0;
+    FilterPlan filt_plan;
+    bool filt_march = false;        // the taps fit the marching kernel
     uint8_t *d_fixed = nullptr;
     double *d_fw = nullptr;
     // hierarchy
@@ -918,6 +920,7 @@ int create_impl(tosp_handle *h, const tosp_problem *pb, const tosp_mg_params *mg
         h->filt_r = 0;
         for (const FilterTap &t : taps)
             h->filt_r = std::max(h->filt_r, std::max(std::abs(t.dx), std::max(std::abs(t.dy), std::abs(t.dz))));
+        h->filt_march = filter_plan(taps, h->filt_plan);
         if (h->ntaps) {
             TRY(dalloc(h, &h->d_taps, h->ntaps));
             CK(cudaMemcpy(h->d_taps, taps.data(), sizeof(FilterTap) * taps.size(), cudaMemcpyHostToDevice));
@@ -995,6 +998,18 @@ int setup_levels(tosp_handle *h) {
         return TOSP_ERR_BREAKDOWN;
     }
     if (!h->small_built) TRY(build_small<T>(h));
+    return TOSP_OK;
+}
+
+// y = filtered x on the density mesh (device vectors, x != y).
+int filter_apply(tosp_handle *h, const double *x, double *y, int trans) {
+    if (h->filt_march)
+        launch_filter_march(x, y, h->d_fw, h->d_fixed, h->filt_plan, h->dens.nelx, h->dens.nely, h->dens.nelz, trans,
+                            h->stream);
+    else
+        launch_filter(x, y, h->d_fw, h->d_fixed, h->d_taps, h->ntaps, h->dens.nelx, h->dens.nely, h->dens.nelz, trans,
+                      0, h->filt_r, h->stream);
+    CKL();
     return TOSP_OK;
 }
 
@@ -1724,9 +1739,7 @@ int tosp_apply_filter(tosp_handle *h, const double *x, double *y, int64_t ndens,
     if (h->opfilter == 0 || h->ntaps == 0) {
         CK(cudaMemcpyAsync(dst, src, sizeof(double) * ndens, cudaMemcpyDefault, h->stream));
     } else {
-        launch_filter(src, dst, h->d_fw, h->d_fixed, h->d_taps, h->ntaps, h->dens.nelx, h->dens.nely, h->dens.nelz,
-                      trans ? 1 : 0, 0, h->filt_r, h->stream);
-        CKL();
+        TRY(filter_apply(h, src, dst, trans ? 1 : 0));
     }
     if (!dout) TRY(store_vec(h, y, dst, ndens));
     return sync(h);
@@ -1759,15 +1772,13 @@ int tosp_grad(tosp_handle *h, const double *u, int64_t nfull, double *fgrad, dou
         TRY(load_vec(h, h->d_ufull, u, nfull));
         du = h->d_ufull;
     }
-    launch_grad(du, h->d_rho, h->d_free_elem, h->d_ke64, h->d_g0, h->fg, h->n, h->p, h->emin, h->E, h->stream);
+    launch_grad(du, h->d_rho, h->d_free_elem, h->d_g0, h->fg, h->n, h->mk64, h->p, h->emin, h->E, h->stream);
     CKL();
     double *dst = dout ? fgrad : h->d_gf;
     if (h->opfilter == 0 || h->ntaps == 0) {
         CK(cudaMemcpyAsync(dst, h->d_g0, sizeof(double) * ndens, cudaMemcpyDeviceToDevice, h->stream));
     } else {
-        launch_filter(h->d_g0, dst, h->d_fw, h->d_fixed, h->d_taps, h->ntaps, h->dens.nelx, h->dens.nely,
-                      h->dens.nelz, 1, 0, h->filt_r, h->stream);
-        CKL();
+        TRY(filter_apply(h, h->d_g0, dst, 1));
     }
     if (!dout) TRY(store_vec(h, fgrad, dst, ndens));
     if (fgrad0) TRY(store_vec(h, fgrad0, h->d_g0, ndens));

@@ -116,8 +116,8 @@ void launch_fine_modal(int n, FineMode mode, const FineArgs<T> &a, const WT *w, 
 void launch_fine_diag(double *y, const double *w, const uint8_t *freemask, const double *ke64, const FineGeom &fg,
                       int n, cudaStream_t st);
 // Sensitivities g0 (I/Grad.m:24-49), zero for elements not in freeDensG.
-void launch_grad(const double *u, const double *rho, const uint8_t *free_elem, const double *kepack,
-                 double *g0, const FineGeom &fg, int n, double p, double emin, double E, cudaStream_t st);
+void launch_grad(const double *u, const double *rho, const uint8_t *free_elem, double *g0, const FineGeom &fg, int n,
+                 const ModalCoef<double> &k, double p, double emin, double E, cudaStream_t st);
 
 // Galerkin coarse element matrices (FP64, 576 per coarse element).
 // Finest coarsening by the sub-cell table (coarse elements whose fine nodes
@@ -232,6 +232,17 @@ void launch_small_cycle(const SmallStep<T> *steps_dev, int nsteps, GridBarrier *
 void launch_filter(const double *x, double *y, const double *wsum, const uint8_t *fixed,
                    const FilterTap *taps_dev, int ntaps, int nelx, int nely, int nelz, int trans,
                    int weights_only, int radius, cudaStream_t st);
+
+// The filter marching along z (cubic cells): all offsets of squared length up to
+// d2, with the weight w[squared length].
+struct FilterPlan {
+    static constexpr int D2MAX = 9;
+    int d2 = 0;
+    double w[D2MAX + 1] = {};
+};
+bool filter_plan(const std::vector<FilterTap> &taps, FilterPlan &pl);
+void launch_filter_march(const double *x, double *y, const double *wsum, const uint8_t *fixed, const FilterPlan &pl,
+                         int nelx, int nely, int nelz, int trans, cudaStream_t st);
 
 // Vector kernels.
 void launch_scatter_free(const double *v, const int64_t *idx, int64_t nfree, double *full, cudaStream_t st);

@@ -10,6 +10,7 @@
 // the child's fixed dofs.  Summing Abar_E over E and zeroing the coarse fixed
 // dofs gives P'AP on the free dofs exactly.  For the apply, the element
 // matrices are assembled into a 27-point node stencil of 3x3 blocks.
+#include "launch.cuh"
 #include "tosp_internal.h"
 
 namespace tosp {
@@ -351,8 +352,8 @@ template void launch_assemble_stencil<float>(const double *, const uint8_t *, co
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(128)
-k_stencil(const T *__restrict__ stv, const T *__restrict__ x, const T *__restrict__ b, const T *__restrict__ invdiag,
-          T *__restrict__ y, Grid g, int mode) {
+k_stencil(const T *__restrict__ stv, const T *x, const T *b, const T *__restrict__ invdiag, T *y, Grid g, int mode) {
+    dep_enter();
     for (int64_t I = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; I < g.nnodes;
          I += (int64_t)gridDim.x * blockDim.x) {
         int xx, yy, zz;
@@ -395,8 +396,8 @@ k_stencil(const T *__restrict__ stv, const T *__restrict__ x, const T *__restric
 // partial rows.
 template <typename T>
 __global__ void __launch_bounds__(256)
-k_stencil_warp(const T *__restrict__ stv, const T *__restrict__ x, const T *__restrict__ b,
-               const T *__restrict__ invdiag, T *__restrict__ y, Grid g, int mode) {
+k_stencil_warp(const T *__restrict__ stv, const T *x, const T *b, const T *__restrict__ invdiag, T *y, Grid g, int mode) {
+    dep_enter();
     const int lane = threadIdx.x & 31;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t I = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; I < g.nnodes; I += nw) {
@@ -437,11 +438,10 @@ void launch_stencil(const T *st_vals, const T *x, const T *b, const T *invdiag, 
     if (node_major) {
         int64_t blocks = (g.nnodes + 7) / 8;   // 8 warps per block
         if (blocks > 65535) blocks = 65535;
-        k_stencil_warp<T><<<(unsigned)blocks, 256, 0, st>>>(st_vals, x, b, invdiag, y, g, mode);
+        launch_dep(k_stencil_warp<T>, (unsigned)blocks, 256, 0, st, st_vals, x, b, invdiag, y, g, mode);
     } else {
-        k_stencil<T><<<grid_for(g.nnodes, 128), 128, 0, st>>>(st_vals, x, b, invdiag, y, g, mode);
+        launch_dep(k_stencil<T>, grid_for(g.nnodes, 128), 128, 0, st, st_vals, x, b, invdiag, y, g, mode);
     }
-    count_launch();
 }
 template void launch_stencil<double>(const double *, const double *, const double *, const double *, double *,
                                      const Grid &, int, bool, cudaStream_t);
@@ -455,12 +455,13 @@ template void launch_stencil<float>(const float *, const float *, const float *,
 // product is skipped).
 template <typename T>
 __global__ void k_jacobi_zero(T *x, const T *b, const T *invd, int64_t n) {
+    dep_enter();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         x[i] = invd[i] * b[i];
 }
 template <typename T>
 void launch_jacobi_zero(T *x, const T *b, const T *invdiag, int64_t n, cudaStream_t st) {
-    k_jacobi_zero<T><<<grid_for(n, 256), 256, 0, st>>>(x, b, invdiag, n); count_launch();
+    launch_dep(k_jacobi_zero<T>, grid_for(n, 256), 256, 0, st, x, b, invdiag, n);
 }
 template void launch_jacobi_zero<double>(double *, const double *, const double *, int64_t, cudaStream_t);
 template void launch_jacobi_zero<float>(float *, const float *, const float *, int64_t, cudaStream_t);
@@ -496,8 +497,9 @@ constexpr int64_t TR_SMALL = 65536;
 // the same bit for bit.
 template <typename T, int C>
 __global__ void __launch_bounds__(C == 1 ? 128 : 256)
-k_prolong(const T *__restrict__ xc, T *__restrict__ xf, const uint8_t *__restrict__ fmf, Grid gf, Grid gc,
+k_prolong(const T *xc, T *xf, const uint8_t *__restrict__ fmf, Grid gf, Grid gc,
           int accumulate) {
+    dep_enter();
     const int64_t n = gf.ndof / C;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t I = C == 3 ? i : i / 3;
@@ -544,10 +546,9 @@ template <typename T>
 void launch_prolong(const T *xc, T *xf, const uint8_t *freemask_f, const Grid &gf, const Grid &gc, bool accumulate,
                     cudaStream_t st) {
     if (gf.nnodes <= TR_SMALL)
-        k_prolong<T, 1><<<grid_for(gf.ndof, 128), 128, 0, st>>>(xc, xf, freemask_f, gf, gc, accumulate ? 1 : 0);
+        launch_dep(k_prolong<T, 1>, grid_for(gf.ndof, 128), 128, 0, st, xc, xf, freemask_f, gf, gc, accumulate ? 1 : 0);
     else
-        k_prolong<T, 3><<<grid_for(gf.nnodes, 256), 256, 0, st>>>(xc, xf, freemask_f, gf, gc, accumulate ? 1 : 0);
-    count_launch();
+        launch_dep(k_prolong<T, 3>, grid_for(gf.nnodes, 256), 256, 0, st, xc, xf, freemask_f, gf, gc, accumulate ? 1 : 0);
 }
 template void launch_prolong<double>(const double *, double *, const uint8_t *, const Grid &, const Grid &, bool,
                                      cudaStream_t);
@@ -558,8 +559,9 @@ template void launch_prolong<float>(const float *, float *, const uint8_t *, con
 // weighted by zero (loads issue together; same sum, same order).
 template <typename T, int C>
 __global__ void __launch_bounds__(C == 1 ? 128 : 256)
-k_restrict(const T *__restrict__ rf, T *__restrict__ bc, const uint8_t *__restrict__ fmc, Grid gf, Grid gc,
-           const T *__restrict__ invdc, T *__restrict__ xc) {
+k_restrict(const T *rf, T *bc, const uint8_t *__restrict__ fmc, Grid gf, Grid gc,
+           const T *__restrict__ invdc, T *xc) {
+    dep_enter();
     const int64_t n = gc.ndof / C;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t J = C == 3 ? i : i / 3;
@@ -607,10 +609,9 @@ template <typename T>
 void launch_restrict(const T *rf, T *bc, const uint8_t *freemask_c, const Grid &gf, const Grid &gc, cudaStream_t st,
                      const T *invd_c, T *xc) {
     if (gc.nnodes <= TR_SMALL)
-        k_restrict<T, 1><<<grid_for(gc.ndof, 128), 128, 0, st>>>(rf, bc, freemask_c, gf, gc, invd_c, xc);
+        launch_dep(k_restrict<T, 1>, grid_for(gc.ndof, 128), 128, 0, st, rf, bc, freemask_c, gf, gc, invd_c, xc);
     else
-        k_restrict<T, 3><<<grid_for(gc.nnodes, 256), 256, 0, st>>>(rf, bc, freemask_c, gf, gc, invd_c, xc);
-    count_launch();
+        launch_dep(k_restrict<T, 3>, grid_for(gc.nnodes, 256), 256, 0, st, rf, bc, freemask_c, gf, gc, invd_c, xc);
 }
 template void launch_restrict<double>(const double *, double *, const uint8_t *, const Grid &, const Grid &,
                                       cudaStream_t, const double *, double *);

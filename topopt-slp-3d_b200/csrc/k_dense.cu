@@ -7,6 +7,7 @@
 // DB with identity) and inverted once per setup in place by a blocked
 // symmetric sweep, so that each cycle's coarse solve is a single FP64 GEMV
 // that runs from L2.
+#include "launch.cuh"
 #include "tosp_internal.h"
 
 namespace tosp {
@@ -378,7 +379,8 @@ int dense_sweep_inverse(double *A, double *work, double *Pinv, int64_t npad, int
 // x = X b (X symmetric, npad x npad; only the first n entries are used).
 template <typename T>
 __global__ void __launch_bounds__(256)
-k_dense_gemv(const double *__restrict__ X, const T *__restrict__ b, T *__restrict__ x, int64_t n, int64_t npad) {
+k_dense_gemv(const double *__restrict__ X, const T *b, T *x, int64_t n, int64_t npad) {
+    dep_enter();
     // Four warps per row (two rows per block), four partial sums per lane:
     // the coarsest system has only a few thousand rows, and with one warp
     // per row the loads in flight were too few to cover the memory latency.
@@ -416,7 +418,7 @@ void launch_dense_solve(const double *X, const T *b, T *x, int64_t n, int64_t np
     int64_t blocks = (n + 1) / 2;
     if (blocks > 2048) blocks = 2048;
     if (blocks < 1) blocks = 1;
-    k_dense_gemv<T><<<(unsigned)blocks, 256, 0, st>>>(X, b, x, n, npad); count_launch();
+    launch_dep(k_dense_gemv<T>, (unsigned)blocks, 256, 0, st, X, b, x, n, npad);
 }
 template void launch_dense_solve<double>(const double *, const double *, double *, int64_t, int64_t, cudaStream_t);
 template void launch_dense_solve<float>(const double *, const float *, float *, int64_t, int64_t, cudaStream_t);

@@ -28,6 +28,7 @@
 #include <cmath>
 
 #include "fine_modal.cuh"
+#include "launch.cuh"
 #include "tosp_internal.h"
 
 namespace tosp {
@@ -165,6 +166,7 @@ k_fine_modal(const FineArgs<T> a, const WT *__restrict__ w, const Grid g, const 
     constexpr int TH = fine_threads<T>, SZ = (int)sizeof(T), UNROLL = fine_unroll(N);
     constexpr bool MASK = MODE == FINE_APPLY || MODE == FINE_RESID || MODE == FINE_DOT;
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    dep_start();
     const int t = threadIdx.x, EY = pl.ey, EX = pl.ex, TY = EY - 1, TX = EX - 1;
     const int PLN = ((EX + 1) * (EY + 1) * 3 * SZ + 15) / 16 * 16 / SZ;
     // factor slots (16-byte pieces first), then the node planes
@@ -244,6 +246,7 @@ k_fine_modal(const FineArgs<T> a, const WT *__restrict__ w, const Grid g, const 
 #pragma unroll
         for (int q = 0; q < 4; ++q) carry[c][q] = T(0);
     }
+    dep_wait();
     if (z0 > 0) stage(z0 - 1);
     stage(z0);
     stage_w(z0 - 1);
@@ -494,8 +497,7 @@ static void launch_mode(const FineArgs<T> &a, const WT *w, const FineGeom &fg, c
     const size_t smem = fine_smem<N, T, WT, MODE>(plan);
     if (smem > 47 * 1024)   // (the kernel has a few static bytes besides)
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kern<<<plan.blocks(), fine_threads<T>, smem, st>>>(a, w, fg.g, fg.nelx_d, fg.nely_d, plan, k);
-    count_launch();
+    launch_dep(kern, plan.blocks(), fine_threads<T>, smem, st, a, w, fg.g, fg.nelx_d, fg.nely_d, plan, k);
 }
 
 template <int N, typename T, typename WT>

@@ -2,6 +2,7 @@
 // boundary conversions.  Dot products use a fixed two-stage reduction tree
 // (RED_BLOCKS partial sums, then one block), so results are bitwise
 // reproducible run to run.
+#include "launch.cuh"
 #include "tosp_internal.h"
 
 namespace tosp {
@@ -31,12 +32,13 @@ void launch_gather_free(const double *full, const int64_t *idx, int64_t nfree, d
 
 template <typename TI, typename TO>
 __global__ void k_convert(const TI *a, TO *b, int64_t n) {
+    dep_enter();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         b[i] = (TO)a[i];
 }
 template <typename TI, typename TO>
 void launch_convert(const TI *a, TO *b, int64_t n, cudaStream_t st) {
-    k_convert<TI, TO><<<gridv(n), 256, 0, st>>>(a, b, n); count_launch();
+    launch_dep(k_convert<TI, TO>, gridv(n), 256, 0, st, a, b, n);
 }
 template void launch_convert<double, float>(const double *, float *, int64_t, cudaStream_t);
 template void launch_convert<float, double>(const float *, double *, int64_t, cudaStream_t);
@@ -106,6 +108,7 @@ __device__ __forceinline__ double sum_partials(const double *partials, int np, d
 }
 
 __global__ void __launch_bounds__(256, 4) k_dot_partial(const double *a, const double *b, int64_t n, double *partials, double *out) {
+    dep_enter();
     __shared__ double sh[32];
     double s = 0.0;
     constexpr int VB8 = 2 * VB;
@@ -122,12 +125,13 @@ __global__ void __launch_bounds__(256, 4) k_dot_partial(const double *a, const d
 }
 
 void launch_dot(const double *a, const double *b, int64_t n, double *partials, double *out, cudaStream_t st) {
-    k_dot_partial<<<RED_BLOCKS, 256, 0, st>>>(a, b, n, partials, out); count_launch();
+    launch_dep(k_dot_partial, RED_BLOCKS, 256, 0, st, a, b, n, partials, out);
 }
 
 // a'b and a'c in one pass over a (partials: 2 * RED_BLOCKS).
 __global__ void __launch_bounds__(256, 4) k_dot2_partial(const double *a, const double *b, const double *c, int64_t n, double *partials,
                                double *out0, double *out1) {
+    dep_enter();
     __shared__ double sh[32];
     double s = 0.0, t = 0.0;
     double av[VB], bv[VB], cv[VB];
@@ -155,7 +159,7 @@ __global__ void __launch_bounds__(256, 4) k_dot2_partial(const double *a, const 
 
 void launch_dot2(const double *a, const double *b, const double *c, int64_t n, double *partials, double *out0,
                  double *out1, cudaStream_t st) {
-    k_dot2_partial<<<RED_BLOCKS, 256, 0, st>>>(a, b, c, n, partials, out0, out1); count_launch();
+    launch_dep(k_dot2_partial, RED_BLOCKS, 256, 0, st, a, b, c, n, partials, out0, out1);
 }
 
 // Scalar slots (see solver.cpp): 0 rho, 1 gamma2 (previous rho), 2 d'q, 3 r'r,
@@ -168,6 +172,7 @@ void launch_dot2(const double *a, const double *b, const double *c, int64_t n, d
 // d32 (optional) receives the new d in FP32, the input of the FP32 product.
 __global__ void k_pcg_direction(double *d, const double *s, double *sold, const double *scal, int64_t n, int mode,
                                 double *x, float *d32) {
+    dep_enter();
     const double beta = mode == 1 ? 0.0 : (mode == 2 ? (scal[0] - scal[5]) / scal[1] : scal[0] / scal[1]);
     const double alpha = scal[6];
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -185,17 +190,18 @@ __global__ void k_pcg_direction(double *d, const double *s, double *sold, const 
 }
 void launch_pcg_direction(double *d, const double *s, double *sold, const double *scal, int64_t n, int mode,
                           double *x, cudaStream_t st, float *d32) {
-    k_pcg_direction<<<gridv(n), 256, 0, st>>>(d, s, sold, scal, n, mode, x, d32); count_launch();
+    launch_dep(k_pcg_direction, gridv(n), 256, 0, st, d, s, sold, scal, n, mode, x, d32);
 }
 
 // x += alpha d with the last iteration's alpha (slot 6).
 __global__ void k_pcg_finish(double *x, const double *d, const double *scal, int64_t n) {
+    dep_enter();
     const double alpha = scal[6];
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         x[i] += alpha * d[i];
 }
 void launch_pcg_finish(double *x, const double *d, const double *scal, int64_t n, cudaStream_t st) {
-    k_pcg_finish<<<gridv(n), 256, 0, st>>>(x, d, scal, n); count_launch();
+    launch_dep(k_pcg_finish, gridv(n), 256, 0, st, x, d, scal, n);
 }
 
 // r -= alpha q (alpha = rho / d'q, kept in slot 6 for the iterate update),
@@ -206,6 +212,7 @@ void launch_pcg_finish(double *x, const double *d, const double *scal, int64_t n
 template <typename TQ>
 __global__ void __launch_bounds__(256, 4) k_pcg_update(double *r, const TQ *q, double *scal, int64_t n, double *partials, float *b0,
                              const float *invd0, float *x0) {
+    dep_enter();
     __shared__ double sh[32];
     const double alpha = scal[0] / scal[2];
     double s = 0.0;
@@ -243,11 +250,11 @@ __global__ void __launch_bounds__(256, 4) k_pcg_update(double *r, const TQ *q, d
 
 void launch_pcg_update(double *r, const double *q, double *scal, double *partials, int64_t n, cudaStream_t st,
                        float *b0, const float *invd0, float *x0) {
-    k_pcg_update<double><<<RED_BLOCKS, 256, 0, st>>>(r, q, scal, n, partials, b0, invd0, x0); count_launch();
+    launch_dep(k_pcg_update<double>, RED_BLOCKS, 256, 0, st, r, q, scal, n, partials, b0, invd0, x0);
 }
 void launch_pcg_update(double *r, const float *q, double *scal, double *partials, int64_t n, cudaStream_t st,
                        float *b0, const float *invd0, float *x0) {
-    k_pcg_update<float><<<RED_BLOCKS, 256, 0, st>>>(r, q, scal, n, partials, b0, invd0, x0); count_launch();
+    launch_dep(k_pcg_update<float>, RED_BLOCKS, 256, 0, st, r, q, scal, n, partials, b0, invd0, x0);
 }
 
 // Residual replacement: r = f - t (t = K x by the FP64 operator), r'r into
@@ -255,6 +262,7 @@ void launch_pcg_update(double *r, const float *q, double *scal, double *partials
 // FP32 right-hand side and first Jacobi iterate as in k_pcg_update.
 __global__ void __launch_bounds__(256, 4) k_replace_residual(const double *f, const double *t, double *r, double *scal, int64_t n,
                                    double *partials, float *b0, const float *invd0, float *x0) {
+    dep_enter();
     __shared__ double sh[32];
     double s = 0.0;
     double fv[VB], tv[VB];
@@ -285,7 +293,7 @@ __global__ void __launch_bounds__(256, 4) k_replace_residual(const double *f, co
 }
 void launch_replace_residual(const double *f, const double *t, double *r, double *scal, double *partials, int64_t n,
                              cudaStream_t st, float *b0, const float *invd0, float *x0) {
-    k_replace_residual<<<RED_BLOCKS, 256, 0, st>>>(f, t, r, scal, n, partials, b0, invd0, x0); count_launch();
+    launch_dep(k_replace_residual, RED_BLOCKS, 256, 0, st, f, t, r, scal, n, partials, b0, invd0, x0);
 }
 
 __global__ void k_set_scalar(double *dst, const double *src) { *dst = *src; }

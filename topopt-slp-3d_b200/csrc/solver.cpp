@@ -18,6 +18,10 @@ using namespace tosp;
 #include <atomic>
 static std::atomic<long long> g_launches{0};
 void tosp::count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
+bool &tosp::dependent_launches() {
+    thread_local bool on = true;
+    return on;
+}
 long long tosp::launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
 namespace {
@@ -1318,6 +1322,7 @@ int tosp::kelem_prod_with_scratch(tosp_handle *h, const double *x, double *y, in
     } while (0)
 
 int tosp::solve_start(tosp_handle *h, const double *x, const double *f) {
+    SharedGpuScope shared_;
     TRY(need_mg(h));
     TRY(need_setup(h));
     TRY(free_to_full(h, x, h->cx, "x"));
@@ -1332,11 +1337,13 @@ int tosp::solve_start(tosp_handle *h, const double *x, const double *f) {
 }
 
 int tosp::solve_step_account(tosp_handle *h) {
+    SharedGpuScope shared_;
     solve_account(h);
     return replace_residual(h);
 }
 
 int tosp::solve_step(tosp_handle *h) {
+    SharedGpuScope shared_;
     TRY(solve_launch_iteration(h));
     TRY(sync(h));
     solve_account(h);
@@ -1346,6 +1353,7 @@ int tosp::solve_step(tosp_handle *h) {
 const SolveState &tosp::solve_state(const tosp_handle *h) { return h->st; }
 
 int tosp::solve_stop(tosp_handle *h, double *x, int32_t *it, double *relres) {
+    SharedGpuScope shared_;
     const int rc = solve_finish(h, it, relres);
     if (rc < 0) return rc;
     TRY(full_to_free(h, h->cx, x, "x"));
@@ -1471,6 +1479,7 @@ int capture_segments(tosp_handle *h, int parity) {
 
 int tosp::batch_tick(const BatchPlan &plan, cudaStream_t main, cudaEvent_t *ev_mem, cudaEvent_t ev_small,
                      std::string &err) {
+    SharedGpuScope shared_;
     const int nmem = (int)plan.mem.size();
     int nseg = -1;
     for (tosp_handle *h : plan.mem) {

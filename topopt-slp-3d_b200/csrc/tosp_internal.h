@@ -12,6 +12,15 @@
 
 namespace tosp {
 
+// Whether launch_dep (launch.cuh) lets a grid start early on this thread; false
+// while a SharedGpuScope lives (the serving loop's calls).
+bool &dependent_launches();
+struct SharedGpuScope {
+    bool was = dependent_launches();
+    SharedGpuScope() { dependent_launches() = false; }
+    ~SharedGpuScope() { dependent_launches() = was; }
+};
+
 // Count of kernel launches issued by this library (all handles, all threads).
 void count_launch();
 long long launch_count();

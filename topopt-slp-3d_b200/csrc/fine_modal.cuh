@@ -31,7 +31,10 @@
 
 namespace tosp {
 
-template <int N> constexpr int modal_moments = N == 3 ? 27 : (N == 2 ? 8 : 1);
+// N: cells per direction, 1 to 3, or 0 for an element whose 27 moments are given
+// (a coarse element, see k_moments.cu).
+template <int N> constexpr int modal_moments = N == 1 ? 1 : (N == 2 ? 8 : 27);
+template <int N> constexpr int modal_values = N == 0 ? 27 : N * N * N;   // given per element
 
 constexpr double MODAL_R3 = 0.57735026918962576451;   // 1 / sqrt(3)
 
@@ -57,8 +60,11 @@ __host__ __device__ constexpr int modal_sd(int k) { return k == 0 ? 1 : 2; }
 // Moments of the factors w (y fastest, then x, then z) in the scaled basis,
 // up to the constant that ModalCoef carries.
 template <int N, typename T>
-__device__ __forceinline__ void modal_weights(const T (&w)[N * N * N], T (&W)[modal_moments<N>]) {
-    if constexpr (N == 1) {
+__device__ __forceinline__ void modal_weights(const T (&w)[modal_values<N>], T (&W)[modal_moments<N>]) {
+    if constexpr (N == 0) {
+#pragma unroll
+        for (int q = 0; q < 27; ++q) W[q] = w[q];
+    } else if constexpr (N == 1) {
         W[0] = w[0];
     } else if constexpr (N == 2) {
         // cell bits in w's order: 1 y, 2 x, 4 z; W's: 1 x, 2 y, 4 z
@@ -102,7 +108,7 @@ __device__ __forceinline__ void modal_gram(const T (&W)[modal_moments<N>], const
     for (int p = 0; p < 8; ++p) {
         if (!in(p)) continue;
         S[p] = W[modal_index<N>(p, p)] * E[p];
-        if constexpr (N > 1) {
+        if constexpr (N != 1) {
 #pragma unroll
             for (int q = 0; q < 8; ++q)
                 if (q != p && in(q)) S[p] += W[modal_index<N>(p, q)] * E[q];
@@ -260,6 +266,56 @@ __device__ __forceinline__ void modal_energies(const T (&m)[3][8], const ModalCo
                 }
 #pragma unroll
         for (int s = 0; s < 27; ++s) q[s] = F[(s / 3 % 3) + 3 * (s % 3) + 9 * (s / 9)];
+    }
+}
+
+// Diagonal of the element matrix, D[a][c] at corner a (1 y, 2 x, 4 z) and
+// component c.  For the derivative along d the products of modes chi, chi' with
+// chi xor chi' = beta add up to H_d[beta], and a corner's value is the sum of
+// sign^beta over beta.
+template <int N, typename T>
+__device__ __forceinline__ void modal_diagonal(const T (&W)[modal_moments<N>], const ModalCoef<T> &k, T (&D)[8][3]) {
+    T H[3][8];
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+            H[d][b] = T(0);
+            if ((b >> d) & 1) continue;
+#pragma unroll
+            for (int p = 0; p < 8; ++p) {
+                if ((p >> d) & 1) continue;
+                if (N == 1 && b) continue;
+                const int n = modal_deg(p) + modal_deg(p ^ b);   // 3^(-n / 2)
+                H[d][b] += T(n == 0 ? 1.0 : (n == 1 ? MODAL_R3 : (n == 2 ? 1.0 / 3.0 : (n == 3 ? MODAL_R3 / 3.0 : 1.0 / 9.0)))) *
+                           W[modal_index<N>(p, p ^ b)];
+            }
+        }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        T f[8];
+#pragma unroll
+        for (int b = 0; b < 8; ++b) f[b] = (k.kt[c] * k.t[c] + k.kn[c]) * H[c][b];
+#pragma unroll
+        for (int kk = 0; kk < 3; ++kk) {
+            const int sc = modal_sc(kk), sd = modal_sd(kk);
+#pragma unroll
+            for (int b = 0; b < 8; ++b) {
+                if (c == sc) f[b] += k.s1[kk] * H[sd][b];
+                if (c == sd) f[b] += k.s2[kk] * k.sr[kk] * H[sc][b];
+            }
+        }
+#pragma unroll
+        for (int bit = 1; bit < 8; bit <<= 1)
+#pragma unroll
+            for (int b = 0; b < 8; ++b)
+                if (!(b & bit)) {
+                    const T e = f[b], o = f[b | bit];
+                    f[b] = e - o;
+                    f[b | bit] = e + o;
+                }
+#pragma unroll
+        for (int a = 0; a < 8; ++a) D[a][c] = f[((a >> 1) & 1) | ((a & 1) << 1) | (a & 4)];
     }
 }
 

@@ -1,37 +1,11 @@
-// Setup and sensitivity kernels of the finest level: the diagonal of K(w), the
-// SIMP factors and the compliance sensitivities.  (The operator itself:
-// k_fine_modal.cu.)
+// SIMP factors and compliance sensitivities of the finest level.  (The operator:
+// k_fine_modal.cu; its diagonal: k_moments.cu.)
 #include <cuda_bf16.h>
 
 #include "fine_modal.cuh"
 #include "tosp_internal.h"
 
 namespace tosp {
-
-// Diagonal of K(w): one thread per element, atomics (setup only).  Reads the
-// row-major packed blocks ke[s*300 + rowmajor(i,i)].
-template <int N>
-__global__ void k_fine_diag(double *__restrict__ y, const double *__restrict__ w, const uint8_t *__restrict__ freemask,
-                            const double *__restrict__ ke, FineGeom fg) {
-    constexpr int NS = N * N * N;
-    const Grid &g = fg.g;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < g.nelem;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int ey = (int)(e % g.nely), ex = (int)((e / g.nely) % g.nelx), ez = (int)(e / ((int64_t)g.nely * g.nelx));
-        for (int i = 0; i < 24; ++i) {
-            const int t = pair_rowmajor(i, i);
-            double d = 0.0;
-            for (int s = 0; s < NS; ++s) {
-                const int sy = s % N, sx = (s / N) % N, sz = s / (N * N);
-                d += w[((int64_t)(ez * N + sz) * fg.nelx_d + (ex * N + sx)) * fg.nely_d + (ey * N + sy)] *
-                     ke[s * KE_PACK + t];
-            }
-            const int a = i / 3, c = i % 3;
-            const int64_t node = ((int64_t)(ez + ((a >> 2) & 1)) * g.nx + (ex + ((a >> 1) & 1))) * g.ny + (ey + (a & 1));
-            if (freemask[3 * node + c]) atomicAdd(&y[3 * node + c], d);
-        }
-    }
-}
 
 static int num_sms() {
     static int n = 0;
@@ -41,16 +15,6 @@ static int num_sms() {
         cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
     }
     return n;
-}
-
-void launch_fine_diag(double *y, const double *w, const uint8_t *freemask, const double *ke64, const FineGeom &fg,
-                      int n, cudaStream_t st) {
-    int64_t blocks = (fg.g.nelem + 255) / 256;
-    if (blocks > 16 * num_sms()) blocks = 16 * num_sms();
-    if (blocks < 1) blocks = 1;
-    if (n == 1) { k_fine_diag<1><<<(unsigned)blocks, 256, 0, st>>>(y, w, freemask, ke64, fg); count_launch(); }
-    else if (n == 2) { k_fine_diag<2><<<(unsigned)blocks, 256, 0, st>>>(y, w, freemask, ke64, fg); count_launch(); }
-    else { k_fine_diag<3><<<(unsigned)blocks, 256, 0, st>>>(y, w, freemask, ke64, fg); count_launch(); }
 }
 
 // ---------------------------------------------------------------------------

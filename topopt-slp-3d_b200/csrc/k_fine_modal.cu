@@ -40,7 +40,7 @@ namespace {
 // cap of 168 spills, 152 against 119 us at 192 x 96 x 96; n = 1 fits in 160:
 // 80 against 95 us).  FP32 takes 128 (a cap of 80 spills: 131 against 85 us).
 template <typename T> constexpr int fine_threads = sizeof(T) == 8 ? 128 : 256;
-constexpr int fine_resident(int n, int elem_bytes) { return n == 1 && elem_bytes == 8 ? 3 : 2; }
+constexpr int fine_resident(int n, int elem_bytes) { return n == 1 && elem_bytes == 8 ? 3 : 2; }   // (n = 0: moments)
 // Layers per loop trip: two for n = 1, whose carried planes change registers
 // instead of being moved (57 against 62 us, 192 x 96 x 96, BF16); the longer
 // bodies of n = 2 and 3 gain nothing or lose (n = 3: 70 against 57 us).
@@ -96,9 +96,15 @@ __device__ __forceinline__ void stage_factors(unsigned char *slots, const WT *w,
             }
         }
 }
+// (N = 0: the 27 moments of an element, `plane` values apart.)
 template <int N, typename T, typename WT, int TH>
 __device__ __forceinline__ void load_factors(const unsigned char *slots, const WT *w, int64_t row, int64_t plane,
-                                             bool in, T (&v)[N * N * N]) {
+                                             bool in, T (&v)[modal_values<N>]) {
+    if constexpr (N == 0) {
+#pragma unroll
+        for (int q = 0; q < 27; ++q) v[q] = in ? (T)__ldg(w + q * plane) : T(0);
+        return;
+    }
     using S = FineSlot<N, WT>;
 #pragma unroll
     for (int sz = 0; sz < N; ++sz)
@@ -222,12 +228,15 @@ k_fine_modal(const FineArgs<T> a, const WT *__restrict__ w, const Grid g, const 
     const bool own = act && i >= 1 && j >= 1;
     const int ni = act ? (i * (EY + 1) + j) * 3 : 0;             // low corner in the staged plane
     const int si = own ? ((i - 1) * TY + (j - 1)) * 3 : 0;       // node in the sums
-    const int64_t wrow = nely_d, wplane = (int64_t)nelx_d * nely_d;
-    const WT *wp = inside ? w + (int64_t)ex * N * wrow + ey * N : w;
+    // cells: rows along y, planes of the density mesh; moments: values one
+    // element apart, the element's 27 `wplane` apart
+    const int64_t wrow = N == 0 ? g.nely : nely_d, wplane = N == 0 ? g.nelem : (int64_t)nelx_d * nely_d;
+    const int64_t wstep = N == 0 ? (int64_t)g.nelx * g.nely : N * wplane;
+    const WT *wp = inside ? w + (int64_t)ex * (N == 0 ? 1 : N) * wrow + ey * (N == 0 ? 1 : N) : w;
     unsigned char *wslot = smem_raw + t * FineSlot<N, WT>::BYTES;
     auto stage_w = [&](int e) {
         if (e >= 0 && e < g.nelz)
-            stage_factors<N, WT, TH>(wslot, wp + (inside ? (int64_t)e * N * wplane : 0), wrow, wplane, inside);
+            stage_factors<N, WT, TH>(wslot, wp + (inside ? e * wstep : 0), wrow, wplane, inside);
     };
 
     auto read_plane = [&](int p, PlaneModes<T> (&m)[3]) {
@@ -317,9 +326,8 @@ k_fine_modal(const FineArgs<T> a, const WT *__restrict__ w, const Grid g, const 
             }
         }
         const bool layer = e < z1 && e >= 0 && e < g.nelz;       // an element layer to compute
-        T wv[N * N * N];
-        if (layer)
-            load_factors<N, T, WT, TH>(wslot, wp + (inside ? (int64_t)e * N * wplane : 0), wrow, wplane, inside, wv);
+        T wv[modal_values<N>];
+        if (layer) load_factors<N, T, WT, TH>(wslot, wp + (inside ? e * wstep : 0), wrow, wplane, inside, wv);
         if (e + 1 < z1) stage_w(e + 1);
         cp_async_commit();
 
@@ -511,6 +519,18 @@ static void launch_n(FineMode mode, const FineArgs<T> &a, const WT *w, const Fin
         case FINE_DOT: return launch_mode<N, T, WT, FINE_DOT>(a, w, fg, plan, k, st);
     }
 }
+
+// A coarse level's product from its moments: the sweeps and the residual.
+template <typename T>
+void launch_moment_product(FineMode mode, const FineArgs<T> &a, const T *mom, const FineGeom &fg, const FinePlan &plan,
+                           const ModalCoef<T> &k, cudaStream_t st) {
+    if (mode == FINE_JACOBI) launch_mode<0, T, T, FINE_JACOBI>(a, mom, fg, plan, k, st);
+    else launch_mode<0, T, T, FINE_RESID>(a, mom, fg, plan, k, st);
+}
+template void launch_moment_product<double>(FineMode, const FineArgs<double> &, const double *, const FineGeom &,
+                                            const FinePlan &, const ModalCoef<double> &, cudaStream_t);
+template void launch_moment_product<float>(FineMode, const FineArgs<float> &, const float *, const FineGeom &,
+                                           const FinePlan &, const ModalCoef<float> &, cudaStream_t);
 
 template <typename T, typename WT>
 void launch_fine_modal(int n, FineMode mode, const FineArgs<T> &a, const WT *w, const FineGeom &fg,

@@ -36,7 +36,30 @@ struct Level {
     void *st = nullptr;        // 27-point stencil (levels 1..L-2), cycle precision
     void *invd = nullptr;      // omega / diag(A), 0 on fixed dofs, cycle precision
     void *b = nullptr, *x = nullptr, *r = nullptr, *t = nullptr;   // cycle vectors
+    // operators from moments (levels >= 1 of a clean hierarchy): the moments, and
+    // on large levels the product that applies them in the cycle precision
+    bool modal = false;
+    double *mom = nullptr;
+    float *mom32 = nullptr;
+    FinePlan plan;
+    FineGeom fg{};
+    uint8_t *fix = nullptr;    // per block of the plan: owns a fixed dof
+    ModalCoef<double> mk64{};
+    ModalCoef<float> mk32{};
 };
+
+ModalCoef<float> to_float(const ModalCoef<double> &k) {
+    ModalCoef<float> f;
+    for (int c = 0; c < 3; ++c) {
+        f.t[c] = (float)k.t[c];
+        f.kt[c] = (float)k.kt[c];
+        f.kn[c] = (float)k.kn[c];
+        f.sr[c] = (float)k.sr[c];
+        f.s1[c] = (float)k.s1[c];
+        f.s2[c] = (float)k.s2[c];
+    }
+    return f;
+}
 
 }  // namespace
 
@@ -91,6 +114,7 @@ struct tosp_handle {
     CoarsePcgWork cpw;
     int *d_info = nullptr;
     bool setup_done = false;
+    bool clean = false;             // every parent of a fixed dof is fixed: coarse operators from moments
     // persistent small-level cycle: first level it covers (-1: off), its grid
     // and three step lists (entered with the first sweep done, from zero, warm)
     // dots the CG wants from the preconditioner's last sweep (cg_iteration)
@@ -269,6 +293,16 @@ void launch_fine(tosp_handle *h, FineMode mode, const FineArgs<T> &args, bool cg
         launch_fine_modal<float, __nv_bfloat16>(h->n, mode, a, h->d_wbf, h->fg, h->plan32, h->mk32, h->stream);
 }
 
+// A sweep or the residual of a level that applies its moments.
+template <typename T>
+void launch_level(tosp_handle *h, Level &L, FineMode mode, const FineArgs<T> &args) {
+    FineArgs<T> a = args;
+    a.fm = L.fm;
+    a.fixed = L.fix;
+    if constexpr (sizeof(T) == 8) launch_moment_product<double>(mode, a, L.mom, L.fg, L.plan, L.mk64, h->stream);
+    else launch_moment_product<float>(mode, a, L.mom32, L.fg, L.plan, L.mk32, h->stream);
+}
+
 // y = K x at the finest level (every dof of y is written).
 template <typename T>
 int fine_apply(tosp_handle *h, const T *x, T *y, bool cg32 = false) {
@@ -320,6 +354,14 @@ int smooth(tosp_handle *h, int l, int niter, bool x_zero, bool first_done = fals
                 launch_fine<T>(h, FINE_JACOBI, a);
                 std::swap(L.x, L.t);
             }
+        } else if (L.modal) {
+            FineArgs<T> a;
+            a.x = (const T *)L.x;
+            a.invd = (const T *)L.invd;
+            a.out = L.t;
+            a.b = b;
+            launch_level<T>(h, L, FINE_JACOBI, a);
+            std::swap(L.x, L.t);
         } else {
             launch_stencil<T>((const T *)L.st, (const T *)L.x, b, (const T *)L.invd, (T *)L.t, L.g, 2, L.nm,
                               h->stream);
@@ -339,6 +381,12 @@ int residual(tosp_handle *h, int l) {
         a.b = (const T *)L.b;
         a.out = L.r;
         launch_fine<T>(h, FINE_RESID, a);
+    } else if (L.modal) {
+        FineArgs<T> a;
+        a.x = (const T *)L.x;
+        a.b = (const T *)L.b;
+        a.out = L.r;
+        launch_level<T>(h, L, FINE_RESID, a);
     } else {
         launch_stencil<T>((const T *)L.st, (const T *)L.x, (const T *)L.b, nullptr, (T *)L.r, L.g, 1, L.nm,
                           h->stream);
@@ -673,6 +721,46 @@ int full_to_free(tosp_handle *h, const double *full, double *v, const char *what
     return TOSP_OK;
 }
 
+void drop_graphs(tosp_handle *h) {
+    for (cudaGraphExec_t &g : h->iter_graph)
+        if (g) {
+            cudaGraphExecDestroy(g);
+            g = nullptr;
+        }
+    for (auto &row : h->seg_graph)
+        for (cudaGraphExec_t &g : row)
+            if (g) {
+                cudaGraphExecDestroy(g);
+                g = nullptr;
+            }
+}
+
+// Buffers of the coarse operators, by how the supports let them be built
+// (h->clean).  Kept when the supports change; what is missing is added.
+int level_buffers(tosp_handle *h) {
+    const int ng = h->ngrids;
+    const size_t tsz = h->precision == TOSP_PREC_FP64 ? 8 : 4;
+    for (int l = 1; l < ng; ++l) {
+        Level &L = h->lev[l];
+        const bool inner = l < ng - 1;
+        L.modal = h->clean && inner && !L.nm;
+        if (h->clean && !L.mom) TRY(dalloc(h, &L.mom, 27 * L.g.nelem));
+        if (L.modal && tsz == 4 && !L.mom32) TRY(dalloc(h, &L.mom32, 27 * L.g.nelem));
+        if (!L.modal && !L.Ae) TRY(dalloc(h, &L.Ae, L.g.nelem * 576));
+        if (!L.modal && inner && !L.st) {
+            uint8_t *sp;
+            TRY(dalloc(h, &sp, (int64_t)tsz * L.g.nnodes * STENCIL_VALS));
+            L.st = sp;
+        }
+        if (L.modal) {
+            if (!L.fix) TRY(dalloc(h, &L.fix, L.plan.blocks()));
+            launch_fine_fixed(L.fm, L.g, L.plan, L.fix, h->stream);
+            CKL();
+        }
+    }
+    return TOSP_OK;
+}
+
 int build_masks(tosp_handle *h, const int64_t *freedofs, int64_t nfree) {
     const Grid &g0 = h->lev[0].g;
     std::vector<int64_t> idx(nfree);
@@ -703,10 +791,20 @@ int build_masks(tosp_handle *h, const int64_t *freedofs, int64_t nfree) {
         launch_fine_fixed(h->lev[0].fm, g0, h->plan32, h->d_fix32, h->stream);
     }
     CKL();
-    for (int l = 0; l + 1 < h->ngrids; ++l)
+    CK(cudaMemsetAsync(h->d_info, 0, sizeof(int), h->stream));
+    for (int l = 0; l + 1 < h->ngrids; ++l) {
         launch_coarse_freemask(h->lev[l].fm, h->lev[l + 1].fm, h->lev[l].g, h->lev[l + 1].g, h->stream);
+        launch_clean(h->lev[l].fm, h->lev[l + 1].fm, h->lev[l].g, h->lev[l + 1].g, h->d_info, h->stream);
+    }
     CKL();
+    int bad = 0;
+    CK(cudaMemcpyAsync(&bad, h->d_info, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    TRY(sync(h));
+    const bool clean = h->mg_ok && !bad;
+    if (clean != h->clean) drop_graphs(h);   // captured iterations hold the other operators
+    h->clean = clean;
     h->setup_done = false;
+    TRY(level_buffers(h));
     return sync(h);
 }
 
@@ -806,16 +904,8 @@ int create_impl(tosp_handle *h, const tosp_problem *pb, const tosp_mg_params *mg
         CK(cudaMemcpy(h->d_cbS, S.data(), sizeof(double) * S.size(), cudaMemcpyHostToDevice));
     }
     {
-        const ModalCoef<double> k = modal_coef(pb->el, pb->eh, pb->ew, pb->nu, h->n);
-        h->mk64 = k;
-        for (int c = 0; c < 3; ++c) {
-            h->mk32.t[c] = (float)k.t[c];
-            h->mk32.kt[c] = (float)k.kt[c];
-            h->mk32.kn[c] = (float)k.kn[c];
-            h->mk32.sr[c] = (float)k.sr[c];
-            h->mk32.s1[c] = (float)k.s1[c];
-            h->mk32.s2[c] = (float)k.s2[c];
-        }
+        h->mk64 = modal_coef(pb->el, pb->eh, pb->ew, pb->nu, h->n);
+        h->mk32 = to_float(h->mk64);
         h->plan64 = fine_plan(g0, h->n, 8);
         h->plan32 = fine_plan(g0, h->n, 4);
     }
@@ -831,11 +921,13 @@ int create_impl(tosp_handle *h, const tosp_problem *pb, const tosp_mg_params *mg
         L.x = vb + tsz * L.g.ndof;
         L.r = vb + 2 * tsz * L.g.ndof;
         L.t = vb + 3 * tsz * L.g.ndof;
-        if (l >= 1) TRY(dalloc(h, &L.Ae, L.g.nelem * 576));
-        if (l >= 1 && l < ng - 1) {
-            uint8_t *sp;
-            TRY(dalloc(h, &sp, (int64_t)tsz * L.g.nnodes * STENCIL_VALS));
-            L.st = sp;
+        if (l >= 1) {
+            const double m = (double)(1 << l);
+            L.nm = L.g.nnodes <= (mg->warp_stencil_max == 0 ? 65536 : mg->warp_stencil_max);
+            L.mk64 = modal_coef(m * pb->el, m * pb->eh, m * pb->ew, pb->nu, 1);
+            L.mk32 = to_float(L.mk64);
+            L.fg.g = L.g;
+            L.plan = fine_plan(L.g, 0, (int)tsz);
         }
         if (l < ng - 1 || !h->mg_ok) {
             uint8_t *ip;
@@ -961,7 +1053,7 @@ int setup_levels(tosp_handle *h) {
     // the V-cycle hierarchy is Galerkin-consistent with the V-cycle's finest
     // operator: FP64 factors for the FP64 path, the BF16-rounded ones for mixed
     const double *wh = h->d_wq ? h->d_wq : h->d_w64;
-    launch_fine_diag(h->d_diag64, wh, h->lev[0].fm, h->d_ke64, h->fg, h->n, h->stream);
+    launch_modal_diag(wh, h->fg, h->n, h->mk64, h->lev[0].fm, h->d_diag64, h->stream);
     CKL();
     if constexpr (sizeof(T) == 8) {
         launch_invert_diag<double>(h->d_diag64, h->lev[0].fm, (double *)h->lev[0].invd, h->mg.omega, nd0, h->stream);
@@ -970,15 +1062,35 @@ int setup_levels(tosp_handle *h) {
         launch_convert<double, float>(h->cs, (float *)h->lev[0].invd, nd0, h->stream);
     }
     CKL();
-    launch_coarse_from_fine_table(wh, h->lev[0].fm, h->d_ke64, h->d_cbS, h->lev[1].Ae, h->fg, h->lev[1].g, h->n,
-                                  h->stream);
+    if (h->clean) {
+        launch_moments_fine(wh, h->fg, h->n, h->lev[1].g, h->lev[1].mom, h->stream);
+        for (int l = 1; l + 1 < ng; ++l)
+            launch_moments_coarse(h->lev[l].mom, h->lev[l].g, h->lev[l + 1].g, h->lev[l + 1].mom, h->stream);
+        for (int l = 1; l < ng; ++l)
+            if (!h->lev[l].modal) launch_elem_matrix(h->lev[l].mom, h->lev[l].g, h->lev[l].mk64, h->lev[l].Ae, h->stream);
+    } else {
+        launch_coarse_from_fine_table(wh, h->lev[0].fm, h->d_ke64, h->d_cbS, h->lev[1].Ae, h->fg, h->lev[1].g, h->n,
+                                      h->stream);
+        for (int l = 1; l < ng - 1; ++l)
+            launch_coarse_from_coarse(h->lev[l].Ae, h->lev[l].fm, h->lev[l].g, h->lev[l + 1].Ae, h->lev[l + 1].g, h->stream);
+    }
     CKL();
     for (int l = 1; l < ng - 1; ++l) {
         Level &L = h->lev[l];
-        const int64_t wmax = h->mg.warp_stencil_max == 0 ? 65536 : h->mg.warp_stencil_max;
-        L.nm = L.g.nnodes <= wmax;
-        launch_assemble_stencil<T>(L.Ae, L.fm, L.g, (T *)L.st, (T *)L.invd, h->mg.omega, L.nm, h->stream);
-        launch_coarse_from_coarse(L.Ae, L.fm, L.g, h->lev[l + 1].Ae, h->lev[l + 1].g, h->stream);
+        if (!L.modal) {
+            launch_assemble_stencil<T>(L.Ae, L.fm, L.g, (T *)L.st, (T *)L.invd, h->mg.omega, L.nm, h->stream);
+            CKL();
+            continue;
+        }
+        CK(cudaMemsetAsync(h->d_diag64, 0, sizeof(double) * L.g.ndof, h->stream));
+        launch_modal_diag(L.mom, L.fg, 0, L.mk64, L.fm, h->d_diag64, h->stream);
+        if constexpr (sizeof(T) == 8) {
+            launch_invert_diag<double>(h->d_diag64, L.fm, (double *)L.invd, h->mg.omega, L.g.ndof, h->stream);
+        } else {
+            launch_invert_diag<double>(h->d_diag64, L.fm, h->cs, h->mg.omega, L.g.ndof, h->stream);
+            launch_convert<double, float>(h->cs, (float *)L.invd, L.g.ndof, h->stream);
+            launch_convert<double, float>(L.mom, L.mom32, 27 * L.g.nelem, h->stream);
+        }
         CKL();
     }
     Level &C = h->lev[ng - 1];

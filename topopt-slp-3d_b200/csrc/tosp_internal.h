@@ -121,9 +121,21 @@ template <typename T, typename WT>
 void launch_fine_modal(int n, FineMode mode, const FineArgs<T> &a, const WT *w, const FineGeom &fg,
                        const FinePlan &plan, const ModalCoef<T> &k, cudaStream_t st);
 
-// y += diag(K(w)) (y zeroed by the caller); ke64: row-major packed blocks.
-void launch_fine_diag(double *y, const double *w, const uint8_t *freemask, const double *ke64, const FineGeom &fg,
-                      int n, cudaStream_t st);
+// Coarse operators from moments (k_moments.cu): mom has 27 values per element,
+// nelem apart.
+template <typename T>
+void launch_moment_product(FineMode mode, const FineArgs<T> &a, const T *mom, const FineGeom &fg, const FinePlan &plan,
+                           const ModalCoef<T> &k, cudaStream_t st);
+void launch_moments_fine(const double *w, const FineGeom &fg, int n, const Grid &gc, double *mom, cudaStream_t st);
+void launch_moments_coarse(const double *mf, const Grid &gf, const Grid &gc, double *mom, cudaStream_t st);
+// diag += diag(K) (zeroed by the caller; 0 on fixed dofs) from the cells (n = 1,
+// 2, 3) or a level's moments (n = 0).
+void launch_modal_diag(const double *w, const FineGeom &fg, int n, const ModalCoef<double> &k, const uint8_t *freemask,
+                       double *diag, cudaStream_t st);
+void launch_elem_matrix(const double *mom, const Grid &g, const ModalCoef<double> &k, double *Ae, cudaStream_t st);
+// *bad = 1 when a fixed dof of the fine grid has a free parent on the coarse one.
+void launch_clean(const uint8_t *fmf, const uint8_t *fmc, const Grid &gf, const Grid &gc, int *bad, cudaStream_t st);
+
 // Sensitivities g0 (I/Grad.m:24-49), zero for elements not in freeDensG.
 void launch_grad(const double *u, const double *rho, const uint8_t *free_elem, double *g0, const FineGeom &fg, int n,
                  const ModalCoef<double> &k, double p, double emin, double E, cudaStream_t st);

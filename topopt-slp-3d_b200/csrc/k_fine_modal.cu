@@ -36,11 +36,18 @@ namespace tosp {
 namespace {
 
 // Threads per block and blocks per SM the registers are capped for.  FP64 keeps
-// 2 x 12 plane modes, 21 modes and 21 gradients in registers (253 for n = 2; a
-// cap of 168 spills, 152 against 119 us at 192 x 96 x 96; n = 1 fits in 160:
-// 80 against 95 us).  FP32 takes 128 (a cap of 80 spills: 131 against 85 us).
+// 2 x 12 plane modes, 21 modes and 21 gradients in registers: n = 1 fits in 168
+// (192 x 96 x 96: 71 against 91 us with two blocks; four blocks 87), the others take
+// 250 (n = 2 capped at 168 spills, 152 us, and with its carried values in shared
+// memory instead runs alone in 110 against 119 us but makes a whole solve 5 %
+// longer).  FP32 takes 128 (three blocks of 80 spill: 131 against 85 us for n = 2).
 template <typename T> constexpr int fine_threads = sizeof(T) == 8 ? 128 : 256;
-constexpr int fine_resident(int n, int elem_bytes) { return n == 1 && elem_bytes == 8 ? 3 : 2; }   // (n = 0: moments)
+constexpr int fine_resident(int n, int elem_bytes) { return n == 1 && elem_bytes == 8 ? 3 : 2; }
+// For n = 3, which otherwise spills, the plane modes and the upper plane's part wait
+// for the next layer in the thread's own shared slots (160 x 80 x 40: FP64 88 ->
+// 70 us, V-cycle 56 -> 52, CG 58 -> 54; a mixed solve 71 -> 67 ms).
+constexpr bool fine_stash(int n) { return n == 3; }
+template <int BYTES> constexpr int FINE_STASH = BYTES == 4 ? 27 : 24;   // values per thread
 // Layers per loop trip: two for n = 1, whose carried planes change registers
 // instead of being moved (57 against 62 us, 192 x 96 x 96, BF16); the longer
 // bodies of n = 2 and 3 gain nothing or lose (n = 3: 70 against 57 us).
@@ -48,6 +55,15 @@ constexpr int fine_unroll(int n) { return n == 1 ? 2 : 1; }
 __device__ __forceinline__ float factor_value(__nv_bfloat16 v) { return __bfloat162float(v); }
 __device__ __forceinline__ float factor_value(float v) { return v; }
 __device__ __forceinline__ double factor_value(double v) { return v; }
+
+// Pitch of a staged row: thread t = i EY + j reads at i pitch + 3 j, which falls on
+// the banks of 3 t (no two alike) when the pitch is 3 EY up to whole rounds of
+// the banks.  With the rows end to end every warp has a conflict, 36 % more
+// shared-memory passes; that shows in the stashing kernels only, and the others
+// keep the registers (n = 1, FP64: 71 against 75 us).
+__host__ __device__ constexpr int fine_pitch(int n, int elem_bytes, int ey) {
+    return fine_stash(n) ? 3 * ey + 128 / elem_bytes : 3 * (ey + 1);
+}
 
 constexpr uint32_t FINE_NONE = 0xffffffffu;   // no value at this place
 constexpr int FINE_NQ = 4;   // plane values staged per thread
@@ -100,39 +116,39 @@ __device__ __forceinline__ void stage_factors(unsigned char *slots, const WT *w,
 template <int N, typename T, typename WT, int TH>
 __device__ __forceinline__ void load_factors(const unsigned char *slots, const WT *w, int64_t row, int64_t plane,
                                              bool in, T (&v)[modal_values<N>]) {
+    using S = FineSlot<N, WT>;
     if constexpr (N == 0) {
 #pragma unroll
         for (int q = 0; q < 27; ++q) v[q] = in ? (T)__ldg(w + q * plane) : T(0);
-        return;
-    }
-    using S = FineSlot<N, WT>;
+    } else {
 #pragma unroll
-    for (int sz = 0; sz < N; ++sz)
+        for (int sz = 0; sz < N; ++sz)
 #pragma unroll
-        for (int sx = 0; sx < N; ++sx)
+            for (int sx = 0; sx < N; ++sx)
 #pragma unroll
-            for (int sy = 0; sy < N / S::CELLS; ++sy) {
-                const int q = (sz * N + sx) * (N / S::CELLS) + sy;
-                T *o = v + q * S::CELLS;
-                const unsigned char *p = slots + q * TH * S::BYTES;
-                if constexpr (!fine_stage_w<N, WT>) {
-                    o[0] = in ? (T)factor_value(__ldg(w + sz * plane + sx * row + sy)) : T(0);
-                } else if constexpr (N == 2 && sizeof(WT) == 2) {
-                    const __nv_bfloat162 c = *reinterpret_cast<const __nv_bfloat162 *>(p);
-                    o[0] = (T)__low2float(c);
-                    o[1] = (T)__high2float(c);
-                } else if constexpr (N == 2 && sizeof(WT) == 4) {
-                    const float2 c = *reinterpret_cast<const float2 *>(p);
-                    o[0] = (T)c.x;
-                    o[1] = (T)c.y;
-                } else if constexpr (N == 2) {
-                    const double2 c = *reinterpret_cast<const double2 *>(p);
-                    o[0] = (T)c.x;
-                    o[1] = (T)c.y;
-                } else {
-                    o[0] = (T)*reinterpret_cast<const WT *>(p);
+                for (int sy = 0; sy < N / S::CELLS; ++sy) {
+                    const int q = (sz * N + sx) * (N / S::CELLS) + sy;
+                    T *o = v + q * S::CELLS;
+                    const unsigned char *p = slots + q * TH * S::BYTES;
+                    if constexpr (!fine_stage_w<N, WT>) {
+                        o[0] = in ? (T)factor_value(__ldg(w + sz * plane + sx * row + sy)) : T(0);
+                    } else if constexpr (N == 2 && sizeof(WT) == 2) {
+                        const __nv_bfloat162 c = *reinterpret_cast<const __nv_bfloat162 *>(p);
+                        o[0] = (T)__low2float(c);
+                        o[1] = (T)__high2float(c);
+                    } else if constexpr (N == 2 && sizeof(WT) == 4) {
+                        const float2 c = *reinterpret_cast<const float2 *>(p);
+                        o[0] = (T)c.x;
+                        o[1] = (T)c.y;
+                    } else if constexpr (N == 2) {
+                        const double2 c = *reinterpret_cast<const double2 *>(p);
+                        o[0] = (T)c.x;
+                        o[1] = (T)c.y;
+                    } else {
+                        o[0] = (T)*reinterpret_cast<const WT *>(p);
+                    }
                 }
-            }
+    }
 }
 
 __device__ __forceinline__ double fine_block_sum(double v, double *sh) {
@@ -157,10 +173,11 @@ constexpr int fine_epi_bytes = MODE == FINE_RESID    ? (int)sizeof(T)
 
 template <int N, typename T, typename WT, int MODE>
 size_t fine_smem(const FinePlan &p) {
-    const size_t pl = (size_t)(p.ex + 1) * (p.ey + 1) * 3;
+    const size_t pl = (size_t)(p.ex + 1) * fine_pitch(N, sizeof(T), p.ey);
     const size_t plane = (pl * sizeof(T) + 15) / 16 * 16;
     return 2 * plane + fine_threads<T> * (2 * 9 * sizeof(T) + 2 * 3 * sizeof(T) + 3 * fine_epi_bytes<T, MODE> +
-                                          (fine_stage_w<N, WT> ? N * N * N * sizeof(WT) : 0));
+                                          (fine_stage_w<N, WT> ? N * N * N * sizeof(WT) : 0) +
+                                          (fine_stash(N) ? FINE_STASH<sizeof(T)> * sizeof(T) : 0));
 }
 
 }  // namespace
@@ -174,12 +191,15 @@ k_fine_modal(const FineArgs<T> a, const WT *__restrict__ w, const Grid g, const 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     dep_start();
     const int t = threadIdx.x, EY = pl.ey, EX = pl.ex, TY = EY - 1, TX = EX - 1;
-    const int PLN = ((EX + 1) * (EY + 1) * 3 * SZ + 15) / 16 * 16 / SZ;
+    const int PITCH = fine_pitch(N, SZ, EY), PLN = ((EX + 1) * PITCH * SZ + 15) / 16 * 16 / SZ;
     // factor slots (16-byte pieces first), then the node planes
     constexpr int WB = fine_stage_w<N, WT> ? N * N * N * (int)sizeof(WT) * TH : 0;
-    T *planes = reinterpret_cast<T *>(smem_raw + WB);            // 2 x PLN
+    constexpr bool STASH = fine_stash(N);
+    constexpr int SB = STASH ? FINE_STASH<SZ> * SZ * TH : 0;
+    T *stash = reinterpret_cast<T *>(smem_raw + WB) + t;         // FINE_STASH x TH
+    T *planes = reinterpret_cast<T *>(smem_raw + WB + SB);       // 2 x PLN
     T *corners = planes + 2 * PLN;                               // 2 x 9 x TH
-    T *sums = corners + 2 * 9 * TH;                              // 2 x 3 x TH, dense over the owned tile
+    T *sums = corners + 2 * 9 * TH;                              // 2 x 3 x TH, rows of 3 TY (STASH: 3 EY)
     double *epd = reinterpret_cast<double *>(sums + 2 * 3 * TH); // FINE_OUT: r, so; FINE_DOT: r (3 x TH each)
     T *ept = MODE == FINE_OUT ? reinterpret_cast<T *>(epd + 6 * TH) : sums + 2 * 3 * TH;
 
@@ -190,7 +210,7 @@ k_fine_modal(const FineArgs<T> a, const WT *__restrict__ w, const Grid g, const 
     // Staging: value f of the (EX + 1) x (EY + 1) x 3 halo of a plane, as its
     // byte offset in the plane.  Values outside the mesh are never copied:
     // their slots of both buffers are cleared here.
-    uint32_t goff[FINE_NQ];
+    uint32_t goff[FINE_NQ], soff[FINE_NQ];
     {
         const int rw = 3 * (EY + 1), n = (EX + 1) * rw;
 #pragma unroll
@@ -199,24 +219,27 @@ k_fine_modal(const FineArgs<T> a, const WT *__restrict__ w, const Grid g, const 
             const int gx = x0 - 1 + row, gv = 3 * (y0 - 1) + col;
             const bool in = f < n && gx >= 0 && gx < g.nx && gv >= 0 && gv < 3 * g.ny;
             goff[q] = in ? (uint32_t)(gx * 3 * g.ny + gv) * SZ : FINE_NONE;
-            if (f < n && !in) planes[f] = planes[PLN + f] = T(0);
+            soff[q] = STASH ? (uint32_t)(row * PITCH + col) : (uint32_t)f;
+            if (f < n && !in) planes[soff[q]] = planes[PLN + soff[q]] = T(0);
         }
     }
     auto stage = [&](int p) {
-        T *dst = planes + (p & 1) * PLN + t;
+        T *dst = planes + (p & 1) * PLN;
         const char *src = reinterpret_cast<const char *>(a.x + p * zs);
 #pragma unroll
         for (int q = 0; q < FINE_NQ; ++q)
-            if (goff[q] != FINE_NONE) cp_async<SZ>(dst + q * TH, src + goff[q], true);
+            if (goff[q] != FINE_NONE) cp_async<SZ>(dst + soff[q], src + goff[q], true);
     };
     // output: value f of the TX x TY x 3 owned values of a plane
     uint32_t ooff[3];
+    int spos[3];                                                 // its place in the sums
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
         const int f = t + q * TH, row = f / (3 * TY), col = f - row * 3 * TY;
         ooff[q] = row < TX && x0 + row < g.nx && 3 * y0 + col < 3 * g.ny
                       ? (uint32_t)((x0 + row) * 3 * g.ny + 3 * y0 + col)
                       : FINE_NONE;
+        spos[q] = STASH ? row * 3 * EY + col : f;
     }
     // blocks without a fixed dof do not read the mask
     const bool fixed = MASK && (!a.fixed || a.fixed[blockIdx.x]);
@@ -226,8 +249,8 @@ k_fine_modal(const FineArgs<T> a, const WT *__restrict__ w, const Grid g, const 
     const bool act = i < EX;
     const bool inside = act && ex >= 0 && ex < g.nelx && ey >= 0 && ey < g.nely;
     const bool own = act && i >= 1 && j >= 1;
-    const int ni = act ? (i * (EY + 1) + j) * 3 : 0;             // low corner in the staged plane
-    const int si = own ? ((i - 1) * TY + (j - 1)) * 3 : 0;       // node in the sums
+    const int ni = act ? i * PITCH + 3 * j : 0;                  // low corner in the staged plane
+    const int si = own ? 3 * ((i - 1) * (STASH ? EY : TY) + (j - 1)) : 0;   // node in the sums
     // cells: rows along y, planes of the density mesh; moments: values one
     // element apart, the element's 27 `wplane` apart
     const int64_t wrow = N == 0 ? g.nely : nely_d, wplane = N == 0 ? g.nelem : (int64_t)nelx_d * nely_d;
@@ -239,9 +262,25 @@ k_fine_modal(const FineArgs<T> a, const WT *__restrict__ w, const Grid g, const 
             stage_factors<N, WT, TH>(wslot, wp + (inside ? e * wstep : 0), wrow, wplane, inside);
     };
 
+    // (STASH) plane modes of component c, then the upper plane's parts
+    constexpr int LV = SZ == 4 ? 5 : 4;
+    auto stash_modes = [&](int c, const PlaneModes<T> &m) {
+        T *o = stash + LV * c * TH;
+        o[0] = m.s;
+        o[TH] = m.x;
+        o[2 * TH] = m.y;
+        o[3 * TH] = m.xy;
+        if constexpr (SZ == 4) o[4 * TH] = m.b;
+    };
+    auto stashed_modes = [&](int c) {
+        const T *o = stash + LV * c * TH;
+        return PlaneModes<T>{SZ == 4 ? o[(LV - 1) * TH] : T(0), o[0], o[TH], o[2 * TH], o[3 * TH]};
+    };
+    T *const stash_top = stash + 3 * LV * TH;
+
     auto read_plane = [&](int p, PlaneModes<T> (&m)[3]) {
         const T *s = planes + (p & 1) * PLN + ni;
-        const int up = act ? 3 * (EY + 1) : 0, hi = act ? 3 : 0;
+        const int up = act ? PITCH : 0, hi = act ? 3 : 0;
 #pragma unroll
         for (int c = 0; c < 3; ++c) m[c] = plane_modes<T>(s[c], s[hi + c], s[up + c], s[up + hi + c]);
     };
@@ -263,6 +302,14 @@ k_fine_modal(const FineArgs<T> a, const WT *__restrict__ w, const Grid g, const 
     cp_async_wait();
     __syncthreads();
     if (z0 > 0) read_plane(z0 - 1, lo);
+    if constexpr (STASH) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            stash_modes(c, lo[c]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) stash_top[(4 * c + q) * TH] = T(0);
+        }
+    }
     __syncthreads();   // the slot of plane z0 - 1 is staged next
 
     uint8_t mask[3] = {1, 1, 1};
@@ -271,14 +318,14 @@ k_fine_modal(const FineArgs<T> a, const WT *__restrict__ w, const Grid g, const 
     for (int e = z0 - 1; e <= z1 + 1; ++e) {
         // epilogue of plane e - 2
         if (e - 2 >= z0) {
-            const T *sp = sums + (e & 1) * 3 * TH + t;
+            const T *sp = sums + (e & 1) * 3 * TH;
             T *out = static_cast<T *>(a.out) + (e - 2) * zs;
             double *out64 = static_cast<double *>(a.out) + (e - 2) * zs;
 #pragma unroll
             for (int q = 0; q < 3; ++q) {
                 const uint32_t o = ooff[q];
                 if (o == FINE_NONE) continue;
-                const T v = sp[q * TH];
+                const T v = sp[spos[q]];
                 const T *et = ept + t + q * TH;
                 if constexpr (MODE == FINE_APPLY) {
                     out[o] = mask[q] ? v : T(0);
@@ -354,16 +401,28 @@ k_fine_modal(const FineArgs<T> a, const WT *__restrict__ w, const Grid g, const 
                 cp[(6 + c) * TH] = p + q;
             };
             if (e + 1 < g.nz) read_plane(e + 1, hi);
+            if constexpr (STASH) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) lo[c] = stashed_modes(c);
+            }
             if (layer) {
                 T m[3][8], r[3][8], W[modal_moments<N>];
 #pragma unroll
                 for (int c = 0; c < 3; ++c) element_modes<T>(lo[c], hi[c], m[c]);
+                if constexpr (STASH) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) stash_modes(c, hi[c]);
+                }
                 modal_weights<N, T>(wv, W);
                 modal_stress<N, T>(m, W, k, r);
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
                     const T rxy = T(MODAL_R3) * r[c][3], rxz = T(MODAL_R3) * r[c][5], ryz = T(MODAL_R3) * r[c][6],
                             rxyz = T(1.0 / 3.0) * r[c][7];
+                    if constexpr (STASH) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) carry[c][q] = stash_top[(4 * c + q) * TH];
+                    }
                     if (corner)
                         put(c, carry[c][0] - r[c][4], carry[c][1] + (r[c][1] - rxz), carry[c][2] + (r[c][2] - ryz),
                             carry[c][3] + (rxy - rxyz));
@@ -375,6 +434,11 @@ k_fine_modal(const FineArgs<T> a, const WT *__restrict__ w, const Grid g, const 
             } else {
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
+                    if constexpr (STASH) {
+                        if (e + 1 < g.nz) stash_modes(c, hi[c]);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) carry[c][q] = stash_top[(4 * c + q) * TH];
+                    }
                     if (corner) put(c, carry[c][0], carry[c][1], carry[c][2], carry[c][3]);
 #pragma unroll
                     for (int q = 0; q < 4; ++q) top[c][q] = T(0);
@@ -382,9 +446,12 @@ k_fine_modal(const FineArgs<T> a, const WT *__restrict__ w, const Grid g, const 
             }
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                if (e + 1 < g.nz) lo[c] = hi[c];
+                if (!STASH && e + 1 < g.nz) lo[c] = hi[c];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) carry[c][q] = top[c][q];
+                for (int q = 0; q < 4; ++q) {
+                    if constexpr (STASH) stash_top[(4 * c + q) * TH] = top[c][q];
+                    else carry[c][q] = top[c][q];
+                }
             }
         }
         cp_async_wait();

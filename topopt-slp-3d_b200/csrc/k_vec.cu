@@ -205,36 +205,34 @@ void launch_pcg_finish(double *x, const double *d, const double *scal, int64_t n
 }
 
 // r -= alpha q (alpha = rho / d'q, kept in slot 6 for the iterate update),
-// r'r into slot 3 and gamma2 = rho (last block).  For the mixed V-cycle (b0
-// given) it also writes the next cycle's FP32 right-hand side b0 = r and, when
-// x0 is given, its first Jacobi iterate x0 = invd0 b0 (the sweep from a zero
-// guess).
-template <typename TQ>
+// r'r into slot 3 and gamma2 = rho (last block).  It also writes the next
+// cycle's first Jacobi iterate x0 = invd0 r in the cycle's precision (the sweep
+// from a zero guess; when x0 is given) and, for the mixed V-cycle, its FP32
+// right-hand side b0 = r.
+template <typename TQ, typename TX>
 __global__ void __launch_bounds__(256, 4) k_pcg_update(double *r, const TQ *q, double *scal, int64_t n, double *partials, float *b0,
-                             const float *invd0, float *x0) {
+                             const TX *invd0, TX *x0) {
     dep_enter();
     __shared__ double sh[32];
     const double alpha = scal[0] / scal[2];
     double s = 0.0;
     double rv[VB];
     TQ qv[VB];
-    float dv[VB];
+    TX dv[VB];
     grid_batched(
         n,
         [&](int k, int64_t i) {
             rv[k] = r[i];
             qv[k] = q[i];
-            if (b0 && x0) dv[k] = invd0[i];
+            if (x0) dv[k] = invd0[i];
         },
         [&](int k, int64_t i) {
             const double ri = rv[k] - alpha * (double)qv[k];
             r[i] = ri;
             s += ri * ri;
-            if (b0) {
-                const float bi = (float)ri;
-                b0[i] = bi;
-                if (x0) x0[i] = dv[k] * bi;
-            }
+            const TX bi = (TX)ri;
+            if (b0) b0[i] = (float)ri;
+            if (x0) x0[i] = dv[k] * bi;
         });
     s = block_sum(s, sh);
     if (threadIdx.x == 0) partials[blockIdx.x] = s;
@@ -249,12 +247,16 @@ __global__ void __launch_bounds__(256, 4) k_pcg_update(double *r, const TQ *q, d
 }
 
 void launch_pcg_update(double *r, const double *q, double *scal, double *partials, int64_t n, cudaStream_t st,
+                       const double *invd0, double *x0) {
+    launch_dep(k_pcg_update<double, double>, RED_BLOCKS, 256, 0, st, r, q, scal, n, partials, nullptr, invd0, x0);
+}
+void launch_pcg_update(double *r, const double *q, double *scal, double *partials, int64_t n, cudaStream_t st,
                        float *b0, const float *invd0, float *x0) {
-    launch_dep(k_pcg_update<double>, RED_BLOCKS, 256, 0, st, r, q, scal, n, partials, b0, invd0, x0);
+    launch_dep(k_pcg_update<double, float>, RED_BLOCKS, 256, 0, st, r, q, scal, n, partials, b0, invd0, x0);
 }
 void launch_pcg_update(double *r, const float *q, double *scal, double *partials, int64_t n, cudaStream_t st,
                        float *b0, const float *invd0, float *x0) {
-    launch_dep(k_pcg_update<float>, RED_BLOCKS, 256, 0, st, r, q, scal, n, partials, b0, invd0, x0);
+    launch_dep(k_pcg_update<float, float>, RED_BLOCKS, 256, 0, st, r, q, scal, n, partials, b0, invd0, x0);
 }
 
 // Residual replacement: r = f - t (t = K x by the FP64 operator), r'r into

@@ -631,12 +631,12 @@ int cycle_fmv(tosp_handle *h, int l, double *out = nullptr) {
     return cycle_vw<T>(h, l, false, false, false, out);
 }
 
-// The mixed CG update can prepare the next cycle's FP32 right-hand side and
-// first Jacobi iterate (V/W cycles with a pre-smoothing sweep).
+// The CG update can prepare the next cycle's (FP32) right-hand side and first
+// Jacobi iterate (V/W cycles with a pre-smoothing sweep).
 bool fused_first_sweep(const tosp_handle *h) { return h->mg.cycle != 2 && h->mg.smoothiter1 >= 1; }
 
 // s = M^{-1} r on full-length FP64 vectors (r, s distinct from the level buffers).
-// prepared (mixed only): lev[0].b = float(r) and, when fused_first_sweep,
+// prepared: lev[0].b = float(r) (mixed) and, when fused_first_sweep,
 // lev[0].x = invD b were written by the CG update.
 int precondition(tosp_handle *h, const double *r, double *s, bool prepared = false) {
     Level &F = h->lev[0];
@@ -650,8 +650,9 @@ int precondition(tosp_handle *h, const double *r, double *s, bool prepared = fal
         // the finest level reads r in place
         void *own_b = F.b;
         F.b = const_cast<double *>(r);
-        int rc = h->mg.cycle == 2 ? cycle_fmv<double>(h, 0, out) : cycle_vw<double>(h, 0, true, h->mg.cycle == 1,
-                                                                                     false, out);
+        const bool first_done = prepared && fused_first_sweep(h);
+        int rc = h->mg.cycle == 2 ? cycle_fmv<double>(h, 0, out)
+                                  : cycle_vw<double>(h, 0, true, h->mg.cycle == 1, first_done, out);
         F.b = own_b;
         if (rc != TOSP_OK) {
             F.x = x0;
@@ -1194,8 +1195,8 @@ int cg_iteration(tosp_handle *h, int mode, int k) {
     const bool alt = h->mg.flexible && (k & 1);
     double *s = alt ? h->cso : h->cs;
     double *s_old = alt ? h->cs : h->cso;
-    // iterations after the first find the V-cycle's input prepared by the
-    // previous update (mixed precision)
+    // iterations after the first find the cycle's input prepared by the
+    // previous update
     // the dots of the new s ride on the preconditioner's last sweep when it
     // writes s (post-smoothing), else they take their own pass
     h->fdot.so = mode == 2 ? s_old : nullptr;
@@ -1203,7 +1204,7 @@ int cg_iteration(tosp_handle *h, int mode, int k) {
     h->fdot.o1 = h->d_scal + 5;
     h->fdot.want = true;
     h->fdot.done = false;
-    const int prc = precondition(h, h->cr, s, mixed && mode != 1);
+    const int prc = precondition(h, h->cr, s, mode != 1);
     h->fdot.want = false;
     TRY(prc);
     if (!h->fdot.done) {
@@ -1212,10 +1213,10 @@ int cg_iteration(tosp_handle *h, int mode, int k) {
     }
     launch_pcg_direction(h->cd, s, nullptr, h->d_scal, nd, mode, h->cx, h->stream, h->cg32 ? h->cd32 : nullptr);
     CKL();
-    const bool first = mixed && fused_first_sweep(h);
+    const bool first = fused_first_sweep(h);
     float *b0 = mixed ? (float *)F.b : nullptr;
-    const float *invd0 = first ? (const float *)F.invd : nullptr;
-    float *x0 = first ? (float *)F.x : nullptr;
+    const float *invd0 = mixed && first ? (const float *)F.invd : nullptr;
+    float *x0 = mixed && first ? (float *)F.x : nullptr;
     if (h->cg32) {
         FineArgs<float> a;
         a.x = h->cd32;
@@ -1231,7 +1232,10 @@ int cg_iteration(tosp_handle *h, int mode, int k) {
         a.r = h->cd;
         a.o0 = h->d_scal + 2;
         launch_fine<double>(h, FINE_DOT, a);
-        launch_pcg_update(h->cr, h->cq, h->d_scal, h->d_partials, nd, h->stream, b0, invd0, x0);
+        if (mixed) launch_pcg_update(h->cr, h->cq, h->d_scal, h->d_partials, nd, h->stream, b0, invd0, x0);
+        else
+            launch_pcg_update(h->cr, h->cq, h->d_scal, h->d_partials, nd, h->stream,
+                              first ? (const double *)F.invd : nullptr, first ? (double *)F.x : nullptr);
     }
     CKL();
     CK(cudaMemcpyAsync(h->h_scal, h->d_scal, sizeof(double) * 8, cudaMemcpyDeviceToHost, h->stream));

@@ -281,9 +281,11 @@ void launch_pcg_direction(double *d, const double *s, double *sold, const double
                           double *x, cudaStream_t st, float *d32 = nullptr);
 void launch_pcg_finish(double *x, const double *d, const double *scal, int64_t n, cudaStream_t st);
 void launch_pcg_update(double *r, const double *q, double *scal, double *partials, int64_t n, cudaStream_t st,
-                       float *b0 = nullptr, const float *invd0 = nullptr, float *x0 = nullptr);
+                       const double *invd0, double *x0);
+void launch_pcg_update(double *r, const double *q, double *scal, double *partials, int64_t n, cudaStream_t st,
+                       float *b0, const float *invd0, float *x0);
 void launch_pcg_update(double *r, const float *q, double *scal, double *partials, int64_t n, cudaStream_t st,
-                       float *b0 = nullptr, const float *invd0 = nullptr, float *x0 = nullptr);
+                       float *b0, const float *invd0, float *x0);
 // r = f - t with r'r into scal[3] (residual replacement of cg_product 1), and
 // the next mixed cycle's input as in launch_pcg_update.
 void launch_replace_residual(const double *f, const double *t, double *r, double *scal, double *partials, int64_t n,

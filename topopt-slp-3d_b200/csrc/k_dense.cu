@@ -7,6 +7,8 @@
 // DB with identity) and inverted once per setup in place by a blocked
 // symmetric sweep, so that each cycle's coarse solve is a single FP64 GEMV
 // that runs from L2.
+#include <algorithm>
+
 #include "launch.cuh"
 #include "tosp_internal.h"
 
@@ -198,6 +200,7 @@ __device__ __forceinline__ void tile_inverse(double (&v)[2][4][2], TileInverse &
 
 __global__ void __launch_bounds__(256) k_sweep_first(const double *A, int64_t npad, double *Pinv, int *info) {
     __shared__ __align__(16) TileInverse w;
+    dep_enter();
     const int t = threadIdx.x;
     double v[2][4][2];
 #pragma unroll
@@ -215,9 +218,10 @@ __global__ void __launch_bounds__(256) k_sweep_first(const double *A, int64_t np
 // (64 x npad each), and the column's new values.  Warp w makes columns 8 w .. + 7.
 constexpr int PR = 16, GS = PR + 4;
 constexpr int PANEL_SMEM = (DB * TS + DB * GS) * (int)sizeof(double);
-__global__ void __launch_bounds__(256) k_sweep_panel(double *A, int64_t npad, int k, const double *__restrict__ Pinv,
-                                                     double *__restrict__ Gt, double *__restrict__ Ct) {
+__global__ void __launch_bounds__(256) k_sweep_panel(double *A, int64_t npad, int k, const double *Pinv, double *Gt,
+                                                     double *Ct) {
     extern __shared__ __align__(16) double sm[];
+    dep_enter();
     double *P = sm, *G = sm + DB * TS;                    // P[q][c], G[q][r]
     const int t = threadIdx.x, i = blockIdx.x / (DB / PR), r0 = i * DB + (int)(blockIdx.x % (DB / PR)) * PR;
     if (i == k) {
@@ -280,12 +284,12 @@ __global__ void __launch_bounds__(256) k_sweep_panel(double *A, int64_t npad, in
 // tile (k + 1, k + 1) and inverts it.
 constexpr int DQ = 16;   // rows of Ct and Gt staged at a time (two stages)
 __global__ void __launch_bounds__(256, 4) k_sweep_update(double *A, int64_t npad, int nt, int k,
-                                                         const double *__restrict__ Gt, const double *__restrict__ Ct,
-                                                         double *Pinv, int *info) {
+                                                         const double *Gt, const double *Ct, double *Pinv, int *info) {
     __shared__ __align__(16) union {
         double st[2][2][DQ * TS];
         TileInverse w;
     } sm;
+    dep_enter();
     const int t = threadIdx.x;
     int i, j;
     if (blockIdx.x == 0) {
@@ -342,6 +346,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_update(double *A, int64_t npad
 // A = -(lower tiles), mirrored.
 __global__ void __launch_bounds__(256) k_sweep_mirror(double *A, int64_t npad) {
     __shared__ double T[DB][DB + 1];
+    dep_enter();
     const int e0 = (int)blockIdx.x, t = threadIdx.x;
     int i = (int)((sqrt(8.0 * e0 + 1.0) - 1.0) * 0.5);
     while ((i + 1) * (i + 2) / 2 <= e0) ++i;
@@ -361,18 +366,25 @@ __global__ void __launch_bounds__(256) k_sweep_mirror(double *A, int64_t npad) {
     }
 }
 
-int dense_sweep_inverse(double *A, double *work, double *Pinv, int64_t npad, int *d_info, cudaStream_t st) {
+// Entries more than `band` from the diagonal are zero on entry.  The Schur
+// complements keep the band, so when block k is swept the row tiles above `hi`
+// still hold their first values, with zeros in column k: their C and G are zero
+// and nothing of them changes.  Leaving them out takes the third to a half of the
+// updates (the same results bit for bit).
+int dense_sweep_inverse(double *A, double *work, double *Pinv, int64_t npad, int64_t band, int *d_info,
+                        cudaStream_t st) {
     const int nt = (int)(npad / DB), tiles = nt * (nt + 1) / 2;
     double *Gt = work, *Ct = work + DB * npad;
     cudaFuncSetAttribute(k_sweep_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, PANEL_SMEM);
     cudaMemsetAsync(d_info, 0, sizeof(int), st);
-    k_sweep_first<<<1, 256, 0, st>>>(A, npad, Pinv, d_info); count_launch();
+    launch_dep(k_sweep_first, 1, 256, 0, st, A, npad, Pinv, d_info);
     for (int k = 0; k < nt; ++k) {
-        k_sweep_panel<<<nt * (DB / PR), 256, PANEL_SMEM, st>>>(A, npad, k, Pinv, Gt, Ct); count_launch();
+        const int hi = (int)std::min<int64_t>(nt - 1, (DB * (int64_t)(k + 1) - 1 + std::max<int64_t>(band, 1)) / DB);
+        launch_dep(k_sweep_panel, (hi + 1) * (DB / PR), 256, PANEL_SMEM, st, A, npad, k, Pinv, Gt, Ct);
         if (nt == 1) break;
-        k_sweep_update<<<1 + tiles, 256, 0, st>>>(A, npad, nt, k, Gt, Ct, Pinv, d_info); count_launch();
+        launch_dep(k_sweep_update, 1 + (hi + 1) * (hi + 2) / 2, 256, 0, st, A, npad, nt, k, Gt, Ct, Pinv, d_info);
     }
-    k_sweep_mirror<<<tiles, 256, 0, st>>>(A, npad); count_launch();
+    launch_dep(k_sweep_mirror, tiles, 256, 0, st, A, npad);
     return 0;
 }
 

@@ -1105,7 +1105,9 @@ int setup_levels(tosp_handle *h) {
     }
     launch_dense_assemble(C.Ae, C.fm, C.g, h->d_Adense, h->npad, h->stream);
     CKL();
-    dense_sweep_inverse(h->d_Adense, h->d_sweep, h->d_pinv, h->npad, h->d_info, h->stream);
+    // dofs of neighbouring nodes: one plane, one row and one node apart at most
+    const int64_t band = 3 * ((int64_t)C.g.nx * C.g.ny + C.g.ny + 1) + 2;
+    dense_sweep_inverse(h->d_Adense, h->d_sweep, h->d_pinv, h->npad, band, h->d_info, h->stream);
     CKL();
     int info = 0;
     CK(cudaMemcpyAsync(&info, h->d_info, sizeof(int), cudaMemcpyDeviceToHost, h->stream));

@@ -183,7 +183,9 @@ void launch_coarse_freemask(const uint8_t *freemask_f, uint8_t *freemask_c, cons
 constexpr int DENSE_BLOCK = 64;
 void launch_dense_assemble(const double *Ae, const uint8_t *freemask, const Grid &g, double *A,
                            int64_t npad, cudaStream_t st);
-int dense_sweep_inverse(double *A, double *work, double *Pinv, int64_t npad, int *d_info, cudaStream_t st);
+// band: an upper bound on |i - j| over the nonzeros (npad: none known).
+int dense_sweep_inverse(double *A, double *work, double *Pinv, int64_t npad, int64_t band, int *d_info,
+                        cudaStream_t st);
 template <typename T>
 void launch_dense_solve(const double *X, const T *b, T *x, int64_t n, int64_t npad, cudaStream_t st);
 

@@ -8,6 +8,7 @@
 // symmetric sweep, so that each cycle's coarse solve is a single FP64 GEMV
 // that runs from L2.
 #include <algorithm>
+#include <vector>
 
 #include "launch.cuh"
 #include "tosp_internal.h"
@@ -47,17 +48,17 @@ void launch_dense_assemble(const double *Ae, const uint8_t *freemask, const Grid
 // Sweeping block k of a symmetric matrix:  P = A_kk,  G_i = A_ik,
 // C_i = G_i P^{-1},
 //   A_ij -= C_i G_j' (i, j != k),  A_ik = C_i,  A_kk = -P^{-1}.
-// After all blocks the array holds -A^{-1}.  Every pivot block is a Schur
+// After all blocks the array holds -A^{-1}, whatever their order.  Every pivot block is a Schur
 // complement of the SPD matrix (a leading-block Cholesky factor exists), so no
 // pivoting is needed.  Only the tiles on and below the diagonal are kept up to
 // date; the last pass mirrors and negates them.
 //
-// Two launches per block of 64: the panel (G and C, stored transposed so that
+// Two launches per step, a block of 64 or two: the panel (G and C, stored transposed so that
 // the update reads rows), and the rank-64 update by 64 x 64 tiles, whose first
-// block takes the next pivot's tile and inverts it while the others work.
+// blocks take the next pivots' tiles and invert them while the others work.
 // With blocks of 32, four launches each and the pivot on its own, the chain of
-// small launches was the time: 1 911 dofs 3.0 -> 1.0 ms, 4 158 dofs
-// 17 -> 4.0 ms (FP64 floor of the half updates, n^3 / 2 FMAs: 0.19 and 1.9 ms).
+// small launches was the time: 1 911 dofs 3.0 -> 1.0 ms, 4 158 dofs 17 -> 4.0 ms
+// one block a step and without regard to the band (see dense_sweep_inverse).
 //
 // The products run as FP64 matrix instructions (8 x 8 x 4): with FMAs and 4 x 4
 // values per thread the shared-memory reads, four wavefronts for a 16-byte load
@@ -198,10 +199,19 @@ __device__ __forceinline__ void tile_inverse(double (&v)[2][4][2], TileInverse &
                 make_double2(-v[f][g][0], -v[f][g][1]);
 }
 
-__global__ void __launch_bounds__(256) k_sweep_first(const double *A, int64_t npad, double *Pinv, int *info) {
+// One step: np pivots k[p], the row tiles a[p] .. b[p] that each touches, and the
+// next step's pivots (-1: none).  Buffers of pivot p: Gt and Ct at 2 p and 2 p + 1
+// times DB npad in the work space, the pivot's inverse at p DB^2 in Pinv.
+struct SweepStep {
+    int np = 1, k[2] = {0, -1}, a[2] = {0, 0}, b[2] = {0, -1}, next[2] = {-1, -1};
+};
+
+__global__ void __launch_bounds__(256) k_sweep_first(const double *A, int64_t npad, const SweepStep s, double *Pinv,
+                                                     int *info) {
     __shared__ __align__(16) TileInverse w;
     dep_enter();
-    const int t = threadIdx.x;
+    const int t = threadIdx.x, k = blockIdx.x ? s.k[1] : s.k[0];
+    A += (int64_t)k * DB * (npad + 1);
     double v[2][4][2];
 #pragma unroll
     for (int f = 0; f < 2; ++f)
@@ -211,19 +221,23 @@ __global__ void __launch_bounds__(256) k_sweep_first(const double *A, int64_t np
             v[f][g][0] = o.x;
             v[f][g][1] = o.y;
         }
-    tile_inverse(v, w, t, 0, Pinv, info);
+    tile_inverse(v, w, t, k * DB, Pinv + blockIdx.x * DB * DB, info);
 }
 
 // PR rows of row tile i of block column k: Gt[q][i] = G_i', Ct[c][i] = C_i'
 // (64 x npad each), and the column's new values.  Warp w makes columns 8 w .. + 7.
 constexpr int PR = 16, GS = PR + 4;
 constexpr int PANEL_SMEM = (DB * TS + DB * GS) * (int)sizeof(double);
-__global__ void __launch_bounds__(256) k_sweep_panel(double *A, int64_t npad, int k, const double *Pinv, double *Gt,
-                                                     double *Ct) {
+__global__ void __launch_bounds__(256) k_sweep_panel(double *A, int64_t npad, const SweepStep s, const double *Pinv,
+                                                     double *work) {
     extern __shared__ __align__(16) double sm[];
     dep_enter();
     double *P = sm, *G = sm + DB * TS;                    // P[q][c], G[q][r]
-    const int t = threadIdx.x, i = blockIdx.x / (DB / PR), r0 = i * DB + (int)(blockIdx.x % (DB / PR)) * PR;
+    const int rows0 = s.b[0] - s.a[0] + 1, row = (int)blockIdx.x / (DB / PR), p = row < rows0 ? 0 : 1, k = p ? s.k[1] : s.k[0];
+    const int t = threadIdx.x, i = p == 0 ? s.a[0] + row : s.a[1] + row - rows0,
+              r0 = i * DB + (int)(blockIdx.x % (DB / PR)) * PR;
+    double *Gt = work + 2 * p * DB * npad, *Ct = Gt + DB * npad;
+    Pinv += p * DB * DB;
     if (i == k) {
         for (int e = t; e < PR * DB; e += 256)
             A[(int64_t)(r0 + e / DB) * npad + k * DB + e % DB] = -Pinv[(r0 - k * DB) * DB + e];
@@ -280,11 +294,18 @@ __global__ void __launch_bounds__(256) k_sweep_panel(double *A, int64_t npad, in
     }
 }
 
-// A_ij -= C_i G_j' for the tiles i >= j outside row and column k.  Block 0 takes
-// tile (k + 1, k + 1) and inverts it.
+// A_ij -= C_i G_j' for the tiles i >= j outside the pivots' rows and columns, for
+// each pivot that touches both rows.  The first np blocks take the next pivots'
+// tiles and invert them.
 constexpr int DQ = 16;   // rows of Ct and Gt staged at a time (two stages)
-__global__ void __launch_bounds__(256, 4) k_sweep_update(double *A, int64_t npad, int nt, int k,
-                                                         const double *Gt, const double *Ct, double *Pinv, int *info) {
+__device__ __forceinline__ void tri_index(int e, int &i, int &j) {
+    i = (int)((sqrt(8.0 * e + 1.0) - 1.0) * 0.5);
+    while ((i + 1) * (i + 2) / 2 <= e) ++i;
+    while (i * (i + 1) / 2 > e) --i;
+    j = e - i * (i + 1) / 2;
+}
+__global__ void __launch_bounds__(256, 4) k_sweep_update(double *A, int64_t npad, const SweepStep s, const double *work,
+                                                         double *Pinv, int *info) {
     __shared__ __align__(16) union {
         double st[2][2][DQ * TS];
         TileInverse w;
@@ -292,40 +313,51 @@ __global__ void __launch_bounds__(256, 4) k_sweep_update(double *A, int64_t npad
     dep_enter();
     const int t = threadIdx.x;
     int i, j;
-    if (blockIdx.x == 0) {
-        i = j = k + 1;
-        if (i >= nt) return;
+    const bool pivot = (int)blockIdx.x < s.np;
+    if (pivot) {
+        i = j = blockIdx.x ? s.next[1] : s.next[0];
+        if (i < 0) return;
     } else {
-        const int e = (int)blockIdx.x - 1;
-        i = (int)((sqrt(8.0 * e + 1.0) - 1.0) * 0.5);
-        while ((i + 1) * (i + 2) / 2 <= e) ++i;
-        while (i * (i + 1) / 2 > e) --i;
-        j = e - i * (i + 1) / 2;
-        if (i == k || j == k || (i == j && i == k + 1)) return;
+        const int e = (int)blockIdx.x - s.np, rows0 = s.b[0] - s.a[0] + 1, tri0 = rows0 * (rows0 + 1) / 2;
+        tri_index(e < tri0 ? e : e - tri0, i, j);
+        const int o = e < tri0 ? s.a[0] : s.a[1];
+        i += o;
+        j += o;
+        if (e >= tri0 && i <= s.b[0]) return;   // (a[0] = 0: listed with the first pivot's)
+        if (i == s.k[0] || j == s.k[0] || i == s.k[1] || j == s.k[1]) return;
+        if (i == j && (i == s.next[0] || i == s.next[1])) return;
     }
+    // the pivots that touch tile (i, j)
+    const bool in0 = j >= s.a[0] && i <= s.b[0], in1 = s.np == 2 && j >= s.a[1] && i <= s.b[1];
+    const int first = in0 ? 0 : 1, chunks = (in0 && in1 ? 2 : 1) * (DB / DQ);
+    if (!in0 && !in1 && !pivot) return;
     auto stage = [&](int c) {
         double *X = sm.st[c & 1][0], *Y = sm.st[c & 1][1];
+        const int p = c < DB / DQ ? first : 1;
+        const double *Gt = work + (int64_t)2 * p * DB * npad + (int64_t)(c % (DB / DQ)) * DQ * npad, *Ct = Gt + DB * npad;
 #pragma unroll
         for (int u = 0; u < DQ * DB / 2 / 256; ++u) {
             const int e = t + 256 * u, q = e / (DB / 2), col = 2 * (e % (DB / 2));
-            dense_cp16(X + q * TS + col, Ct + (int64_t)(c * DQ + q) * npad + i * DB + col);
-            dense_cp16(Y + q * TS + col, Gt + (int64_t)(c * DQ + q) * npad + j * DB + col);
+            dense_cp16(X + q * TS + col, Ct + (int64_t)q * npad + i * DB + col);
+            dense_cp16(Y + q * TS + col, Gt + (int64_t)q * npad + j * DB + col);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     double acc[2][4][2] = {};
-    stage(0);
-#pragma unroll
-    for (int c = 0; c < DB / DQ; ++c) {
-        if (c + 1 < DB / DQ) {
-            stage(c + 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (in0 || in1) {
+        stage(0);
+#pragma unroll 1
+        for (int c = 0; c < chunks; ++c) {
+            if (c + 1 < chunks) {
+                stage(c + 1);
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+            }
+            __syncthreads();
+            tile_mma(sm.st[c & 1][0], sm.st[c & 1][1], DQ, t, acc);
+            __syncthreads();
         }
-        __syncthreads();
-        tile_mma(sm.st[c & 1][0], sm.st[c & 1][1], DQ, t, acc);
-        __syncthreads();
     }
 #pragma unroll
     for (int f = 0; f < 2; ++f)
@@ -340,7 +372,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep_update(double *A, int64_t npad
             acc[f][g][0] = o.x;
             acc[f][g][1] = o.y;
         }
-    if (blockIdx.x == 0) tile_inverse(acc, sm.w, t, i * DB, Pinv, info);
+    if (pivot) tile_inverse(acc, sm.w, t, i * DB, Pinv + blockIdx.x * DB * DB, info);
 }
 
 // A = -(lower tiles), mirrored.
@@ -366,23 +398,54 @@ __global__ void __launch_bounds__(256) k_sweep_mirror(double *A, int64_t npad) {
     }
 }
 
-// Entries more than `band` from the diagonal are zero on entry.  The Schur
-// complements keep the band, so when block k is swept the row tiles above `hi`
-// still hold their first values, with zeros in column k: their C and G are zero
-// and nothing of them changes.  Leaving them out takes the third to a half of the
-// updates (the same results bit for bit).
+// The order of the pivots.  Entries more than `band` from the diagonal are zero on
+// entry, and the Schur complements keep the band: a pivot k with all lower blocks
+// swept touches the row tiles up to hi(k), one with all higher blocks swept those
+// down to lo(k); the others hold zeros in column k and nothing of them changes.  So
+// the sweep runs from both ends at once, two pivots a step, as long as neither
+// touches the other (tiles that both touch take both updates), and then through
+// what is left between, one a step, touching the lower part and, from where the
+// upper part begins to couple, all.  That shortens the chain of steps, which is
+// the time of small systems, and the updates, which are that of large ones: 1 911
+// dofs (30 blocks, a band of 5) take 18 steps instead of 30, a whole setup 0.66 ms
+// instead of 1.20; 4 158 dofs 2.1 for 4.4 ms, 8 619 dofs 6.5 for 26.8 (with the band
+// alone 1.02, 3.3 and 13.6).
 int dense_sweep_inverse(double *A, double *work, double *Pinv, int64_t npad, int64_t band, int *d_info,
                         cudaStream_t st) {
     const int nt = (int)(npad / DB), tiles = nt * (nt + 1) / 2;
-    double *Gt = work, *Ct = work + DB * npad;
+    const int64_t bw = std::min<int64_t>(std::max<int64_t>(band, 1), npad);
+    auto hi = [&](int k) { return (int)std::min<int64_t>(nt - 1, (DB * (int64_t)(k + 1) - 1 + bw) / DB); };
+    auto lo = [&](int k) { return (int)(std::max<int64_t>(0, DB * (int64_t)k - bw) / DB); };
+    int m = 0;   // steps of two pivots
+    while (m < nt - 1 - m && hi(m) < nt - 1 - m && m < lo(nt - 1 - m)) ++m;
+    std::vector<SweepStep> steps;
+    for (int q = 0; q < m; ++q) {
+        SweepStep s;
+        s.np = 2;
+        s.k[0] = q;
+        s.b[0] = hi(q);
+        s.k[1] = nt - 1 - q;
+        s.a[1] = lo(s.k[1]);
+        s.b[1] = nt - 1;
+        steps.push_back(s);
+    }
+    for (int k = m; k < nt - m; ++k) {
+        SweepStep s;
+        s.k[0] = k;
+        s.b[0] = k >= lo(nt - m) ? nt - 1 : hi(k);
+        steps.push_back(s);
+    }
+    for (size_t q = 0; q + 1 < steps.size(); ++q)
+        for (int p = 0; p < steps[q + 1].np; ++p) steps[q].next[p] = steps[q + 1].k[p];
     cudaFuncSetAttribute(k_sweep_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, PANEL_SMEM);
     cudaMemsetAsync(d_info, 0, sizeof(int), st);
-    launch_dep(k_sweep_first, 1, 256, 0, st, A, npad, Pinv, d_info);
-    for (int k = 0; k < nt; ++k) {
-        const int hi = (int)std::min<int64_t>(nt - 1, (DB * (int64_t)(k + 1) - 1 + std::max<int64_t>(band, 1)) / DB);
-        launch_dep(k_sweep_panel, (hi + 1) * (DB / PR), 256, PANEL_SMEM, st, A, npad, k, Pinv, Gt, Ct);
+    launch_dep(k_sweep_first, steps[0].np, 256, 0, st, A, npad, steps[0], Pinv, d_info);
+    for (const SweepStep &s : steps) {
+        const int r0 = s.b[0] - s.a[0] + 1, r1 = s.np == 2 ? s.b[1] - s.a[1] + 1 : 0;
+        launch_dep(k_sweep_panel, (r0 + r1) * (DB / PR), 256, PANEL_SMEM, st, A, npad, s, Pinv, work);
         if (nt == 1) break;
-        launch_dep(k_sweep_update, 1 + (hi + 1) * (hi + 2) / 2, 256, 0, st, A, npad, nt, k, Gt, Ct, Pinv, d_info);
+        launch_dep(k_sweep_update, s.np + r0 * (r0 + 1) / 2 + r1 * (r1 + 1) / 2, 256, 0, st, A, npad, s, work, Pinv,
+                   d_info);
     }
     launch_dep(k_sweep_mirror, tiles, 256, 0, st, A, npad);
     return 0;

@@ -953,8 +953,8 @@ int create_impl(tosp_handle *h, const tosp_problem *pb, const tosp_mg_params *mg
         TRY(dalloc(h, &w.iters, 1));
     } else if (h->mg_ok) {
         TRY(dalloc(h, &h->d_Adense, h->npad * h->npad));
-        TRY(dalloc(h, &h->d_sweep, 2 * DENSE_BLOCK * h->npad));
-        TRY(dalloc(h, &h->d_pinv, DENSE_BLOCK * DENSE_BLOCK));
+        TRY(dalloc(h, &h->d_sweep, 4 * DENSE_BLOCK * h->npad));
+        TRY(dalloc(h, &h->d_pinv, 2 * DENSE_BLOCK * DENSE_BLOCK));
     }
     TRY(dalloc(h, &h->d_info, 1));
     // densities

@@ -178,7 +178,7 @@ void launch_coarse_freemask(const uint8_t *freemask_f, uint8_t *freemask_c, cons
 
 // Coarsest direct solve: dense SPD matrix (padded to a multiple of DENSE_BLOCK,
 // fixed dofs decoupled with a unit diagonal), explicit inverse in place by a
-// blocked symmetric sweep (work: 2 x DENSE_BLOCK x npad, Pinv: DENSE_BLOCK^2),
+// blocked symmetric sweep (work: 4 x DENSE_BLOCK x npad, Pinv: 2 x DENSE_BLOCK^2),
 // GEMV.
 constexpr int DENSE_BLOCK = 64;
 void launch_dense_assemble(const double *Ae, const uint8_t *freemask, const Grid &g, double *A,

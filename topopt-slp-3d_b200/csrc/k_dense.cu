@@ -5,8 +5,8 @@
 // (I/SetupGMG.m:51-59, I/VCycle.m:40).  Here the coarsest matrix is assembled
 // densely (fixed dofs decoupled with a unit diagonal, padded to a multiple of
 // DB with identity) and inverted once per setup in place by a blocked
-// symmetric sweep, so that each cycle's coarse solve is a single FP64 GEMV
-// that runs from L2.
+// symmetric sweep, so that each cycle's coarse solve is an FP64 GEMV, from L2
+// when it fits (k_dense_gemv) or from half of the matrix (k_dense_symv).
 #include <algorithm>
 #include <vector>
 
@@ -488,14 +488,119 @@ k_dense_gemv(const double *__restrict__ X, const T *b, T *x, int64_t n, int64_t 
     }
 }
 
+// The same from the lower tiles alone, for matrices that L2 does not keep: each is
+// read once, for its own rows and, transposed, for its mirror image's.  A block
+// takes up to SYM_CH tiles of a tile row: the sums of the tiles' columns go out
+// by tile, those of its rows by block, and k_dense_symv_sum adds them up in a fixed
+// order.  Half the bytes against a second launch and the partial sums: 4 158 dofs
+// (138 MB) 17 us less of an FP64 iteration and 12 of a mixed one, 6 591 dofs 23,
+// 9 126 dofs 51; 2 535 dofs (51 MB) 1 us more, 1 911 nothing.  So the line lies at half of L2.
+constexpr int SYM_CH = 4;
+// Partial sums (vectors of npad): 0 .. nt - 1 the column sums of tile row i, then
+// the row sums of chunk c.
+int64_t dense_partials(int64_t npad) { return npad / DB + (npad / DB + SYM_CH - 1) / SYM_CH; }
+
 template <typename T>
-void launch_dense_solve(const double *X, const T *b, T *x, int64_t n, int64_t npad, cudaStream_t st) {
+__global__ void __launch_bounds__(256, 2) k_dense_symv(const double *X, const T *b, double *part, int64_t n, int64_t npad) {
+    __shared__ double xi[DB], xj[SYM_CH][DB], cs[SYM_CH][8][DB];
+    dep_enter();
+    const int t = threadIdx.x, l = t & 31, w = t >> 5, nt = (int)(npad / DB);
+    // tile rows SYM_CH q .. + 3 have q + 1 blocks each
+    static_assert(SYM_CH == 4, "the index below");
+    int q = (int)((sqrt(1.0 + 2.0 * blockIdx.x) - 1.0) * 0.5);
+    while (2 * (q + 1) * (q + 2) <= (int)blockIdx.x) ++q;
+    while (2 * q * (q + 1) > (int)blockIdx.x) --q;
+    const int rem = (int)blockIdx.x - 2 * q * (q + 1), i = SYM_CH * q + rem / (q + 1), c = rem % (q + 1);
+    const int j0 = SYM_CH * c, j1 = min(i + 1, j0 + SYM_CH);
+    auto value = [&](int64_t d) { return d < n ? (double)b[d] : 0.0; };
+    {
+        const int jj = t / DB, r = t % DB;
+        if (j0 + jj < j1) xj[jj][r] = value((int64_t)(j0 + jj) * DB + r);
+        if (t < DB) xi[t] = value((int64_t)i * DB + t);
+    }
+    __syncthreads();
+    double racc[8] = {};
+#pragma unroll
+    for (int jj = 0; jj < SYM_CH; ++jj) {
+        if (j0 + jj >= j1) break;
+        const double *p = X + ((int64_t)i * DB + 8 * w) * npad + (int64_t)(j0 + jj) * DB + 2 * l;
+        double2 v[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) v[r] = *reinterpret_cast<const double2 *>(p + r * npad);
+        const double b0 = xj[jj][2 * l], b1 = xj[jj][2 * l + 1];
+        double c0 = 0.0, c1 = 0.0;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const double u = xi[8 * w + r];
+            racc[r] += v[r].x * b0 + v[r].y * b1;
+            c0 += v[r].x * u;
+            c1 += v[r].y * u;
+        }
+        *reinterpret_cast<double2 *>(&cs[jj][w][2 * l]) = make_double2(c0, c1);
+    }
+    // the eight rows over the lanes: halving exchanges leave row l / 4 in lane l
+#pragma unroll
+    for (int h = 4; h > 0; h >>= 1) {
+        const bool up = l & (4 * h);
+#pragma unroll
+        for (int r = 0; r < h; ++r) {
+            const double keep = up ? racc[r + h] : racc[r], give = up ? racc[r] : racc[r + h];
+            racc[r] = keep + __shfl_xor_sync(0xffffffffu, give, 4 * h);
+        }
+    }
+    racc[0] += __shfl_xor_sync(0xffffffffu, racc[0], 2);
+    racc[0] += __shfl_xor_sync(0xffffffffu, racc[0], 1);
+    if ((l & 3) == 0) part[(int64_t)(nt + c) * npad + (int64_t)i * DB + 8 * w + (l >> 2)] = racc[0];
+    __syncthreads();
+    const int jj = t / DB, r = t % DB;
+    if (j0 + jj < j1 && j0 + jj != i) {
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s += cs[jj][k][r];
+        part[(int64_t)i * npad + (int64_t)(j0 + jj) * DB + r] = s;
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_dense_symv_sum(const double *part, T *x, int64_t n, int64_t npad) {
+    __shared__ double sh[8][32];
+    dep_enter();
+    const int t = threadIdx.x, r = t & 31, w = t >> 5, nt = (int)(npad / DB);
+    const int64_t d = (int64_t)blockIdx.x * 32 + r;
+    const int k = (int)(d / DB), chunks = k / SYM_CH + 1;
+    double s = 0.0;
+#pragma unroll 4
+    for (int q = w; q < chunks; q += 8) s += part[(int64_t)(nt + q) * npad + d];
+#pragma unroll 4
+    for (int q = k + 1 + w; q < nt; q += 8) s += part[(int64_t)q * npad + d];
+    sh[w][r] = s;
+    __syncthreads();
+    if (w == 0 && d < n) {
+        s = 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) s += sh[q][r];
+        x[d] = (T)s;
+    }
+}
+
+static bool dense_symmetric(int64_t npad) { return npad * npad * (int64_t)sizeof(double) > (64 << 20); }
+
+template <typename T>
+void launch_dense_solve(const double *X, const T *b, T *x, int64_t n, int64_t npad, double *work, cudaStream_t st) {
+    if (dense_symmetric(npad)) {
+        const int nt = (int)(npad / DB), q = nt / SYM_CH, rest = nt % SYM_CH;   // full groups of tile rows
+        launch_dep(k_dense_symv<T>, 2 * q * (q + 1) + rest * (q + 1), 256, 0, st, X, b, work, n, npad);
+        launch_dep(k_dense_symv_sum<T>, (unsigned)(npad / 32), 256, 0, st, work, x, n, npad);
+        return;
+    }
     int64_t blocks = (n + 1) / 2;
     if (blocks > 2048) blocks = 2048;
     if (blocks < 1) blocks = 1;
     launch_dep(k_dense_gemv<T>, (unsigned)blocks, 256, 0, st, X, b, x, n, npad);
 }
-template void launch_dense_solve<double>(const double *, const double *, double *, int64_t, int64_t, cudaStream_t);
-template void launch_dense_solve<float>(const double *, const float *, float *, int64_t, int64_t, cudaStream_t);
+template void launch_dense_solve<double>(const double *, const double *, double *, int64_t, int64_t, double *,
+                                         cudaStream_t);
+template void launch_dense_solve<float>(const double *, const float *, float *, int64_t, int64_t, double *,
+                                        cudaStream_t);
 
 }  // namespace tosp

@@ -404,7 +404,8 @@ int coarse_solve(tosp_handle *h) {
         CKL();
         return TOSP_OK;
     }
-    launch_dense_solve<T>(h->d_Adense, (const T *)C.b, (T *)C.x, C.g.ndof, h->npad, h->stream);
+    launch_dense_solve<T>(h->d_Adense, (const T *)C.b, (T *)C.x, C.g.ndof, h->npad, h->d_sweep,
+                          h->stream);
     CKL();
     return TOSP_OK;
 }
@@ -953,7 +954,7 @@ int create_impl(tosp_handle *h, const tosp_problem *pb, const tosp_mg_params *mg
         TRY(dalloc(h, &w.iters, 1));
     } else if (h->mg_ok) {
         TRY(dalloc(h, &h->d_Adense, h->npad * h->npad));
-        TRY(dalloc(h, &h->d_sweep, 4 * DENSE_BLOCK * h->npad));
+        TRY(dalloc(h, &h->d_sweep, std::max<int64_t>(4 * DENSE_BLOCK, dense_partials(h->npad)) * h->npad));
         TRY(dalloc(h, &h->d_pinv, 2 * DENSE_BLOCK * DENSE_BLOCK));
     }
     TRY(dalloc(h, &h->d_info, 1));

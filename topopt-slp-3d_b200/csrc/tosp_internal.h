@@ -187,7 +187,9 @@ void launch_dense_assemble(const double *Ae, const uint8_t *freemask, const Grid
 int dense_sweep_inverse(double *A, double *work, double *Pinv, int64_t npad, int64_t band, int *d_info,
                         cudaStream_t st);
 template <typename T>
-void launch_dense_solve(const double *X, const T *b, T *x, int64_t n, int64_t npad, cudaStream_t st);
+void launch_dense_solve(const double *X, const T *b, T *x, int64_t n, int64_t npad, double *work, cudaStream_t st);
+// Partial sums of the solve from the lower tiles, in vectors of npad (in `work`).
+int64_t dense_partials(int64_t npad);
 
 // Persistent small-level cycle (k_small.cu): the steps of a V/W cycle below a
 // level, resolved to buffers on the host, run by one cooperative kernel with a

@@ -11,6 +11,7 @@
 // dofs gives P'AP on the free dofs exactly.  For the apply, the element
 // matrices are assembled into a 27-point node stencil of 3x3 blocks.
 #include "launch.cuh"
+#include "stencil.cuh"
 #include "tosp_internal.h"
 
 namespace tosp {
@@ -401,45 +402,33 @@ k_stencil(const T *__restrict__ stv, const T *x, const T *b, const T *__restrict
     }
 }
 
-// Small levels: one warp per node over the node-major stencil.  Lane o < 27
-// applies offset o's 3x3 block (nine contiguous values: the warp reads the
-// node's 243 values as one contiguous run), then the warp sums the three
-// partial rows.
+// Small levels: one warp per node over the node-major stencil (stencil.cuh).  The
+// stencil is from the setup, which ends with a synchronisation: a grid that starts
+// before its predecessor is done reads its first nodes' values ahead of the wait.
+// All 18 loads of a lane have to be in flight: held to the registers of five (FP64)
+// or six blocks an SM the compiler spreads them out, and 64 x 32 x 32 W takes 5.1 - 5.5
+// ms instead of 4.9 (a lane per offset: 5.2).
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 5)
 k_stencil_warp(const T *__restrict__ stv, const T *x, const T *b, const T *__restrict__ invdiag, T *y, Grid g, int mode) {
-    dep_enter();
+    dep_start();
     const int lane = threadIdx.x & 31;
+    const bool out = lane == 0 || lane == 3 || lane == 6;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t I = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; I < g.nnodes; I += nw) {
-        T a0 = 0, a1 = 0, a2 = 0;
-        if (lane < 27) {
-            int xx, yy, zz;
-            node_xyz(I, g.ny, g.nx, xx, yy, zz);
-            const int oy = lane % 3 - 1, ox = (lane / 3) % 3 - 1, oz = lane / 9 - 1;
-            const int jx = xx + ox, jy = yy + oy, jz = zz + oz;
-            if (jx >= 0 && jx < g.nx && jy >= 0 && jy < g.ny && jz >= 0 && jz < g.nz) {
-                const int64_t J = I + ((int64_t)oz * g.nx + ox) * g.ny + oy;
-                const T x0 = x[3 * J], x1 = x[3 * J + 1], x2 = x[3 * J + 2];
-                const T *s = stv + I * STENCIL_VALS + lane * 9;
-                a0 = s[0] * x0 + s[1] * x1 + s[2] * x2;
-                a1 = s[3] * x0 + s[4] * x1 + s[5] * x2;
-                a2 = s[6] * x0 + s[7] * x1 + s[8] * x2;
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-            a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-            a2 += __shfl_xor_sync(0xffffffffu, a2, o);
-        }
-        if (lane < 3) {
-            const T a = lane == 0 ? a0 : (lane == 1 ? a1 : a2);
-            const int64_t d = 3 * I + lane;
-            if (mode == 0) y[d] = a;
-            else if (mode == 1) y[d] = b[d] - a;
-            else y[d] = x[d] + invdiag[d] * (b[d] - a);
-        }
+    int64_t I = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    T s[9];
+    if (I < g.nnodes) stencil_load<T>(stv + I * STENCIL_VALS, lane, s);
+    dep_wait();
+    while (I < g.nnodes) {
+        int xx, yy, zz;
+        node_xyz(I, g.ny, g.nx, xx, yy, zz);
+        const int64_t d = 3 * I + lane / 3;
+        const T bd = out && mode ? b[d] : T(0), xd = out && mode == 2 ? x[d] : T(0),
+                id = out && mode == 2 ? invdiag[d] : T(0);
+        const T a = stencil_apply<T>(s, [&](int e) { return x[e]; }, (int)I, xx, yy, zz, g, lane);
+        if (out) y[d] = mode == 0 ? a : (mode == 1 ? bd - a : xd + id * (bd - a));
+        I += nw;
+        if (I < g.nnodes) stencil_load<T>(stv + I * STENCIL_VALS, lane, s);
     }
 }
 

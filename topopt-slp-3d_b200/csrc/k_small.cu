@@ -9,7 +9,7 @@
 // once (SmallStep list, rebuilt after each hierarchy setup) and the kernel walks
 // the list with a grid barrier between steps.  Each step's arithmetic is that of
 // the standalone kernel it replaces (k_stencil_warp, k_restrict, k_prolong,
-// k_jacobi, k_dense_gemv), so the results are the same.
+// k_jacobi; k_dense_gemv up to the order of its sums), so the results are the same.
 //
 // Vectors written by one step and read by a later one are loaded with
 // ld.global.cg (L2, coherent across the grid after the barrier's acquire);
@@ -19,6 +19,7 @@
 // skips its first arrival can be set from the host (tosp_inject_wait_fault),
 // so tests make the wait run out without faulting or hanging the GPU.
 #include "grid_sync.cuh"
+#include "stencil.cuh"
 #include "tosp_internal.h"
 
 namespace tosp {
@@ -40,39 +41,21 @@ __device__ __forceinline__ T ldc(const T *p) {
     return __ldcg(p);
 }
 
-// k_stencil_warp's arithmetic: lane o < 27 applies the node's block for
-// offset o, the warp sums the partial rows.
+// k_stencil_warp's arithmetic.
 template <typename T>
 __device__ void step_stencil(const SmallStep<T> &s, int64_t warp, int64_t nwarps, int lane) {
     const Grid g = s.g;
+    const bool out = lane == 0 || lane == 3 || lane == 6;
     for (int64_t I = warp; I < g.nnodes; I += nwarps) {
-        T a0 = 0, a1 = 0, a2 = 0;
-        if (lane < 27) {
-            int xx, yy, zz;
-            small_node_xyz(I, g.ny, g.nx, xx, yy, zz);
-            const int oy = lane % 3 - 1, ox = (lane / 3) % 3 - 1, oz = lane / 9 - 1;
-            const int jx = xx + ox, jy = yy + oy, jz = zz + oz;
-            if (jx >= 0 && jx < g.nx && jy >= 0 && jy < g.ny && jz >= 0 && jz < g.nz) {
-                const int64_t J = I + ((int64_t)oz * g.nx + ox) * g.ny + oy;
-                const T x0 = ldc(s.x + 3 * J), x1 = ldc(s.x + 3 * J + 1), x2 = ldc(s.x + 3 * J + 2);
-                const T *sv = s.st + I * STENCIL_VALS + lane * 9;
-                a0 = __ldg(sv + 0) * x0 + __ldg(sv + 1) * x1 + __ldg(sv + 2) * x2;
-                a1 = __ldg(sv + 3) * x0 + __ldg(sv + 4) * x1 + __ldg(sv + 5) * x2;
-                a2 = __ldg(sv + 6) * x0 + __ldg(sv + 7) * x1 + __ldg(sv + 8) * x2;
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-            a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-            a2 += __shfl_xor_sync(0xffffffffu, a2, o);
-        }
-        if (lane < 3) {
-            const T a = lane == 0 ? a0 : (lane == 1 ? a1 : a2);
-            const int64_t d = 3 * I + lane;
-            if (s.mode == 1) s.y[d] = ldc(s.b + d) - a;
-            else s.y[d] = ldc(s.x + d) + __ldg(s.invd + d) * (ldc(s.b + d) - a);
-        }
+        int xx, yy, zz;
+        small_node_xyz(I, g.ny, g.nx, xx, yy, zz);
+        const int64_t d = 3 * I + lane / 3;
+        const T b = out ? ldc(s.b + d) : T(0), x = out && s.mode != 1 ? ldc(s.x + d) : T(0),
+                id = out && s.mode != 1 ? __ldg(s.invd + d) : T(0);
+        T sv[9];
+        stencil_load<T>(s.st + I * STENCIL_VALS, lane, sv);
+        const T a = stencil_apply<T>(sv, [&](int e) { return ldc(s.x + e); }, (int)I, xx, yy, zz, g, lane);
+        if (out) s.y[d] = s.mode == 1 ? b - a : x + id * (b - a);
     }
 }
 
@@ -155,7 +138,7 @@ __device__ void step_prolong(const SmallStep<T> &s, int64_t t0, int64_t nt) {
     }
 }
 
-// k_dense_gemv's arithmetic: warp per row, four partial sums.
+// x = X b: warp per row, four partial sums.
 template <typename T>
 __device__ void step_dense(const SmallStep<T> &s, int64_t warp, int64_t nwarps, int lane) {
     const int64_t n = s.n, npad = s.npad;

@@ -115,16 +115,6 @@ struct TileInverse {
     double R[2][SB * TS], QR[SB * TS], Q[SB][SB];   // QR: -Q R
 };
 
-// 1 / d from the hardware's approximation q (about 20 bits): with e = 1 - d q,
-// 1 / d = q / (1 - e) = q (1 + e + e^2 + ...), cut after e^2: a shorter
-// chain than a division, to within the last bits.
-__device__ __forceinline__ double series_rcp(double d) {
-    double q;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(q) : "d"(d));
-    const double e = fma(-d, q, 1.0);
-    return fma(q, fma(e, e, e), q);
-}
-
 // Inverse of the symmetric 8 x 8 block at R[.][p0 + .] by one warp: lane l holds
 // (l / 4, 2 (l % 4)) and the element to its right.
 __device__ __forceinline__ void block_inverse(const double *R, double (&Q)[SB][SB], int p0, int dof0, int *info) {
@@ -138,7 +128,7 @@ __device__ __forceinline__ void block_inverse(const double *R, double (&Q)[SB][S
         const double c1 = __shfl_sync(0xffffffffu, v1, 4 * p + (l & 3));
         if (l == 0 && !(d > 0.0)) atomicCAS(info, 0, 1 + dof0 + p0 + p);
         // (products before the reciprocal: the chain from pivot to pivot is the time)
-        const double q = series_rcp(d), f0 = fr * c0, f1 = fr * c1;
+        const double q = 1.0 / d, f0 = fr * c0, f1 = fr * c1;
         v0 = r == p ? (c == p ? -q : c0 * q) : (c == p ? fr * q : fma(-f0, q, v0));
         v1 = r == p ? (c + 1 == p ? -q : c1 * q) : (c + 1 == p ? fr * q : fma(-f1, q, v1));
     }

@@ -208,7 +208,7 @@ k_fine_modal(const FineArgs<T> a, const WT *__restrict__ w, const Grid g, const 
     const int64_t zs = (int64_t)3 * g.nx * g.ny;                 // values per node plane
 
     // Staging: value f of the (EX + 1) x (EY + 1) x 3 halo of a plane, as its
-    // byte offset in the plane.  Values outside the mesh are never copied:
+    // place in the plane.  Values outside the mesh are never copied:
     // their slots of both buffers are cleared here.
     uint32_t goff[FINE_NQ], soff[FINE_NQ];
     {
@@ -218,14 +218,14 @@ k_fine_modal(const FineArgs<T> a, const WT *__restrict__ w, const Grid g, const 
             const int f = t + q * TH, row = f / rw, col = f - row * rw;
             const int gx = x0 - 1 + row, gv = 3 * (y0 - 1) + col;
             const bool in = f < n && gx >= 0 && gx < g.nx && gv >= 0 && gv < 3 * g.ny;
-            goff[q] = in ? (uint32_t)(gx * 3 * g.ny + gv) * SZ : FINE_NONE;
+            goff[q] = in ? (uint32_t)(gx * 3 * g.ny + gv) : FINE_NONE;
             soff[q] = STASH ? (uint32_t)(row * PITCH + col) : (uint32_t)f;
             if (f < n && !in) planes[soff[q]] = planes[PLN + soff[q]] = T(0);
         }
     }
     auto stage = [&](int p) {
         T *dst = planes + (p & 1) * PLN;
-        const char *src = reinterpret_cast<const char *>(a.x + p * zs);
+        const T *src = a.x + p * zs;
 #pragma unroll
         for (int q = 0; q < FINE_NQ; ++q)
             if (goff[q] != FINE_NONE) cp_async<SZ>(dst + soff[q], src + goff[q], true);

@@ -537,7 +537,7 @@ def profile_kernels(args):
     s.KelemProd(r)       # one FP64 product (the outer CG's operator)
     s.MGCycle(r)         # one V-cycle: two launches of the V-cycle's finest operator
     if args.cg_product:
-        s.KelemProdCG32(r)   # one launch of the CG's tensor-core product
+        s.KelemProdCG32(r)   # one launch of the CG's FP32 product
     if args.profile_solve:
         u, it, rr, rc = s.SolveMG(np.zeros(pb.f.size), pb.f)   # one full mixed solve
         print("solve iterations", it)
@@ -561,7 +561,7 @@ def main():
     ap.add_argument("--flexible", type=int, default=1, help="flexible (Polak-Ribiere) CG beta in both arms")
     ap.add_argument("--cg-product", type=int, default=1, choices=[0, 1],
                     help="mg.cg_product of the headline mixed arm (the other value is timed beside it): 0 FP64 "
-                         "product every CG iteration, 1 tensor-core product with FP64 residual replacement")
+                         "product every CG iteration, 1 FP32 product with FP64 residual replacement")
     ap.add_argument("--slp", default="", choices=["", "config0", "config3"],
                     help="full SLP loop: config0 = 48x24x24 cantilever, FP64, 20 iterations; config3 = 160x80x40 "
                          "bridge (reference axes), MR 3, mixed precision, 100 iterations + GradProj")
@@ -777,25 +777,25 @@ def main():
     achcg = bytescg / (ms_opcg * 1e-3) / 1e9
     ach64 = bytes64 / (ms_op64 * 1e-3) / 1e9
     ach64_tf = flops / (ms_op64 * 1e-3) / 1e12
-    fma_exec = nel * (2148 if n == 2 else 300 * (n ** 3 + 2))      # FMAs the FP64 kernel executes per launch
     share32 = applies32 * ms_op32 / (total_ms / args.steps)
     sharecg = appliescg * ms_opcg / (total_ms / args.steps)
     share64 = applies64 * ms_op64 / (total_ms / args.steps)
     rf64 = {"bound": "hbm", "achieved": round(ach64, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
             "frac": round(ach64 / peaks["hbm_gbs"], 4), "traffic": traffic.get("fp64_operator_bytes_per_launch"),
-            "kernel": "k_fine_apply64<2> (outer-CG FP64 operator)", "algorithmic_bytes_per_launch": bytes64,
-            "ms_per_launch": round(ms_op64, 4), "peak_source": peak_kind,
-            "fp64_pipe": {"executed_fma_per_launch": fma_exec,
-                          "achieved_tflops": round(2 * fma_exec / (ms_op64 * 1e-3) / 1e12, 2),
-                          "nominal_peak_tflops": 37.0}}
+            "kernel": f"k_fine_modal<{n},double> (FP64 operator)", "algorithmic_bytes_per_launch": bytes64,
+            "ms_per_launch": round(ms_op64, 4), "peak_source": peak_kind}
+    fp64_inst = traffic.get("fp64_operator_instructions_per_launch")
+    if fp64_inst:      # FP64 instructions of all threads, against one FMA instruction per lane and clock
+        rf64["fp64_pipe"] = {"instructions_per_launch": fp64_inst,
+                             "achieved_tera_per_s": round(fp64_inst / (ms_op64 * 1e-3) / 1e12, 2),
+                             "nominal_peak_tera_per_s": 18.5}
     rf32 = {"bound": "hbm", "achieved": round(ach32, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
             "frac": round(ach32 / peaks["hbm_gbs"], 4), "traffic": traffic.get("fp32_operator_bytes_per_launch"),
-            "kernel": f"k_fine_apply_tc<{n}> (V-cycle operator, tcgen05 sub-cell block products)"
-                      if (n * pb.nely) % 2 == 0 else "k_fine_apply<float,bf16> (V-cycle operator)",
+            "kernel": f"k_fine_modal<{n},float,bf16> (V-cycle operator)",
             "algorithmic_bytes_per_launch": bytes32, "ms_per_launch": round(ms_op32, 4), "peak_source": peak_kind}
     rfcg = {"bound": "hbm", "achieved": round(achcg, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
             "frac": round(achcg / peaks["hbm_gbs"], 4), "traffic": traffic.get("cg32_operator_bytes_per_launch"),
-            "kernel": f"k_fine_apply_tc<{n},float> (CG product of cg_product 1, FP32 factors)",
+            "kernel": f"k_fine_modal<{n},float,float> (CG product of cg_product 1, FP32 factors)",
             "algorithmic_bytes_per_launch": bytescg, "ms_per_launch": round(ms_opcg, 4), "peak_source": peak_kind}
     # the dominant kernel of the timed step carries the contract's roofline
     ranked = sorted([(share64, rf64), (share32, rf32), (sharecg, rfcg)], key=lambda t: -t[0])

@@ -14,20 +14,37 @@ static unsigned gridv(int64_t n) {
     return (unsigned)b;
 }
 
-__global__ void k_scatter(const double *v, const int64_t *idx, int64_t nfree, double *full) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nfree; i += (int64_t)gridDim.x * blockDim.x)
-        full[idx[i]] = v[i];
+// Free-dof vectors to and from full-length ones, by dof: pos[d] is the place of dof
+// d among the (ascending) free dofs, FREE_NONE on fixed dofs.  Both sides are read and
+// written in order, and the fixed dofs' zeros go out with the rest.  A list of the
+// free dofs in 64 bits instead takes 8 more bytes per dof and call and a pass that
+// clears the vector first.  A block takes FREE_CHUNK dofs, each thread four, whose
+// places it reads ahead of the wait (they are from tosp_create / tosp_set_freedofs).
+// KelemProd, 192 x 96 x 96 MR 2: 184 -> 151 us; 16 x 8 x 8: 22.9 -> 16.7.
+constexpr int FREE_CHUNK = 1024;
+template <bool TO_FULL>
+__global__ void __launch_bounds__(256) k_free(const double *src, const uint32_t *__restrict__ pos, int64_t ndof, double *dst) {
+    dep_start();
+    uint32_t p[4];
+    const int64_t d0 = blockIdx.x * (int64_t)FREE_CHUNK + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) p[k] = d0 + 256 * k < ndof ? pos[d0 + 256 * k] : FREE_NONE;
+    dep_wait();
+    double v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = p[k] != FREE_NONE ? src[TO_FULL ? p[k] : d0 + 256 * k] : 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int64_t d = d0 + 256 * k;
+        if (TO_FULL && d < ndof) dst[d] = v[k];
+        if (!TO_FULL && p[k] != FREE_NONE) dst[p[k]] = v[k];
+    }
 }
-void launch_scatter_free(const double *v, const int64_t *idx, int64_t nfree, double *full, cudaStream_t st) {
-    k_scatter<<<gridv(nfree), 256, 0, st>>>(v, idx, nfree, full); count_launch();
+void launch_scatter_free(const double *v, const uint32_t *pos, int64_t ndof, double *full, cudaStream_t st) {
+    launch_dep(k_free<true>, (unsigned)((ndof + FREE_CHUNK - 1) / FREE_CHUNK), 256, 0, st, v, pos, ndof, full);
 }
-
-__global__ void k_gather(const double *full, const int64_t *idx, int64_t nfree, double *v) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nfree; i += (int64_t)gridDim.x * blockDim.x)
-        v[i] = full[idx[i]];
-}
-void launch_gather_free(const double *full, const int64_t *idx, int64_t nfree, double *v, cudaStream_t st) {
-    k_gather<<<gridv(nfree), 256, 0, st>>>(full, idx, nfree, v); count_launch();
+void launch_gather_free(const double *full, const uint32_t *pos, int64_t ndof, double *v, cudaStream_t st) {
+    launch_dep(k_free<false>, (unsigned)((ndof + FREE_CHUNK - 1) / FREE_CHUNK), 256, 0, st, full, pos, ndof, v);
 }
 
 template <typename TI, typename TO>

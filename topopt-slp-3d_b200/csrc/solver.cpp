@@ -78,7 +78,7 @@ struct tosp_handle {
     FineGeom fg{};
     Grid dens{};               // density (= design) mesh as a grid of elements
     int64_t nfree = 0;
-    int64_t *d_freeidx = nullptr;
+    uint32_t *d_freepos = nullptr;   // place of each dof among the free ones
     // constants
     double *d_ke64 = nullptr;       // blocks packed per s (coarse build, Grad)
     double *d_cbS = nullptr;        // sub-cell Galerkin table of the finest coarsening
@@ -702,8 +702,7 @@ int free_to_full(tosp_handle *h, const double *v, double *full, const char *what
         TRY(load_vec(h, h->d_stage_a, v, h->nfree));
         src = h->d_stage_a;
     }
-    CK(cudaMemsetAsync(full, 0, sizeof(double) * h->fg.g.ndof, h->stream));
-    launch_scatter_free(src, h->d_freeidx, h->nfree, full, h->stream);
+    launch_scatter_free(src, h->d_freepos, h->fg.g.ndof, full, h->stream);
     CKL();
     return TOSP_OK;
 }
@@ -712,12 +711,12 @@ int full_to_free(tosp_handle *h, const double *full, double *v, const char *what
     bool dev = false;
     TRY(arg_location(h, v, what, &dev));
     if (dev) {
-        launch_gather_free(full, h->d_freeidx, h->nfree, v, h->stream);
+        launch_gather_free(full, h->d_freepos, h->fg.g.ndof, v, h->stream);
         CKL();
         return TOSP_OK;
     }
     TRY(ensure_stage(h, h->nfree));
-    launch_gather_free(full, h->d_freeidx, h->nfree, h->d_stage_b, h->stream);
+    launch_gather_free(full, h->d_freepos, h->fg.g.ndof, h->d_stage_b, h->stream);
     CKL();
     TRY(store_vec(h, v, h->d_stage_b, h->nfree));
     return TOSP_OK;
@@ -765,7 +764,11 @@ int level_buffers(tosp_handle *h) {
 
 int build_masks(tosp_handle *h, const int64_t *freedofs, int64_t nfree) {
     const Grid &g0 = h->lev[0].g;
-    std::vector<int64_t> idx(nfree);
+    if (g0.ndof >= FREE_NONE) {   // (a vector of so many dofs is 34 GB)
+        h->err = "more than 2^32 - 2 dofs";
+        return TOSP_ERR_UNSUPPORTED;
+    }
+    std::vector<uint32_t> pos(g0.ndof, FREE_NONE);
     std::vector<uint8_t> fm(g0.ndof, 0);
     int64_t prev = -1;
     for (int64_t i = 0; i < nfree; ++i) {
@@ -779,12 +782,12 @@ int build_masks(tosp_handle *h, const int64_t *freedofs, int64_t nfree) {
             return TOSP_ERR_BAD_ARG;
         }
         prev = d;
-        idx[i] = d;
+        pos[d] = (uint32_t)i;
         fm[d] = 1;
     }
-    if (h->d_freeidx == nullptr || h->nfree < nfree) TRY(dalloc(h, &h->d_freeidx, nfree));
+    if (h->d_freepos == nullptr) TRY(dalloc(h, &h->d_freepos, g0.ndof));
     h->nfree = nfree;
-    CK(cudaMemcpy(h->d_freeidx, idx.data(), sizeof(int64_t) * nfree, cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(h->d_freepos, pos.data(), sizeof(uint32_t) * g0.ndof, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(h->lev[0].fm, fm.data(), g0.ndof, cudaMemcpyHostToDevice));
     if (!h->d_fix64) TRY(dalloc(h, &h->d_fix64, h->plan64.blocks()));
     launch_fine_fixed(h->lev[0].fm, g0, h->plan64, h->d_fix64, h->stream);
@@ -1421,11 +1424,10 @@ int tosp::kelem_prod_with_scratch(tosp_handle *h, const double *x, double *y, in
     }
     TRY(check_len(h, nfree, h->nfree, "x"));
     TRY(need_setup(h));
-    CK(cudaMemsetAsync(xfull, 0, sizeof(double) * h->fg.g.ndof, h->stream));
-    launch_scatter_free(x, h->d_freeidx, h->nfree, xfull, h->stream);
+    launch_scatter_free(x, h->d_freepos, h->fg.g.ndof, xfull, h->stream);
     CKL();
     TRY(fine_apply64(h, xfull, yfull));
-    launch_gather_free(yfull, h->d_freeidx, h->nfree, y, h->stream);
+    launch_gather_free(yfull, h->d_freepos, h->fg.g.ndof, y, h->stream);
     CKL();
     return sync(h);
 }

@@ -270,8 +270,10 @@ void launch_filter_march(const double *x, double *y, const double *wsum, const u
                          int nelx, int nely, int nelz, int trans, cudaStream_t st);
 
 // Vector kernels.
-void launch_scatter_free(const double *v, const int64_t *idx, int64_t nfree, double *full, cudaStream_t st);
-void launch_gather_free(const double *full, const int64_t *idx, int64_t nfree, double *v, cudaStream_t st);
+// (pos: the place of each dof among the free ones, FREE_NONE on fixed dofs)
+constexpr uint32_t FREE_NONE = 0xffffffffu;
+void launch_scatter_free(const double *v, const uint32_t *pos, int64_t ndof, double *full, cudaStream_t st);
+void launch_gather_free(const double *full, const uint32_t *pos, int64_t ndof, double *v, cudaStream_t st);
 template <typename TI, typename TO>
 void launch_convert(const TI *a, TO *b, int64_t n, cudaStream_t st);
 // Deterministic dot products: out[0] = sum a*b (fixed reduction tree).
